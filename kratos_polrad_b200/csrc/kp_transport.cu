@@ -806,12 +806,20 @@ k_forward( const __grid_constant__ fwd_params_t P )
 // serves the ray, the round and the tally.  Measured against the selects, at
 // 1e6 rays' packets: inclination 60, azimuth 0 (96^3 root) 10.09 -> 7.03 ms;
 // 3e5 packets obliquely (52.5, 25) 4.44 -> 3.92 ms; along x 5.99 -> 5.84 ms
-// (there the deposits' atomics are what is left).
+// (there the deposits' atomics were what was left).
+// Deposits: a 64-bit atomic instruction of 32 lanes to 32 pixels took 35 L1
+// wavefronts, and the eight of a deposit 60% of the L1's data pipe.  The warp
+// stages its rays' contributions in shared memory and four lanes add the four
+// components of one ray, one 32-byte sector; zeros (V, where the light was
+// never circular) are not added.  Along x 5.84 -> 3.74 ms, with float tallies
+// and their carries (whose atomics return) 6.15 -> 1.99 ms.
 template< int TALLY, int MODE, bool XZ >
 __global__ void __launch_bounds__( 256, MODE == 2 ? 3 : KP_PEEL_MINB )
 k_peel( const __grid_constant__ fwd_params_t P )
 {
     __shared__ unsigned long long cnt_s[ KP_NCOUNTERS ];
+    struct stage_t { float4 v[ 32 ]; int2 pix[ 32 ]; };
+    __shared__ stage_t stage[ MODE == 0 || MODE == 3 ? 8 : 1 ];   // one per warp
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     if( threadIdx.x < KP_NCOUNTERS ) cnt_s[ threadIdx.x ] = 0;
@@ -889,31 +897,51 @@ k_peel( const __grid_constant__ fwd_params_t P )
 
         if( run == PH_EMIT )
         {
-            if( phase != PH_EMIT ) continue;
             const int leader = __ffs( m_fetch ) - 1;
-            n_seg_done += pk;
             if constexpr( MODE == 0 || MODE == 3 )
-            {
-                const bool dep = task >= 0 && ptau <= P.tau_cut;
+            {   // deposits of the rays that just ended (after_crossing's), by the
+                // whole warp: staged in shared memory, then four lanes add the
+                // four components of one ray
+                const bool ended = phase == PH_EMIT && task >= 0;
+                const bool dep = ended && ptau <= P.tau_cut;
+                const unsigned m_dep = __ballot_sync( FULL, dep );
                 float att = -1.0f;                    // MODE 3: -1 marks a ray beyond the cut
+                stage_t & st = stage[ threadIdx.x >> 5 ];
                 if( dep )
-                {   // deposit of the ray that just ended (after_crossing's)
+                {
                     const task_dep_t o = load_task_deposit( P.pq, task );
                     att = __fmul_rn( o.w, ( float ) phys::kp_exp_neg( -( double ) ptau ) );
-                    deposit_pixel< TALLY >( P, o.pix, o.cpix, __fmul_rn( att, o.I ),
-                                            __fmul_rn( att, o.Q ), __fmul_rn( att, o.U ),
-                                            __fmul_rn( att, o.V ) );
+                    const int k = __popc( m_dep & ( ( 1u << lane ) - 1u ) );
+                    st.v[ k ] = make_float4( __fmul_rn( att, o.I ), __fmul_rn( att, o.Q ),
+                                             __fmul_rn( att, o.U ), __fmul_rn( att, o.V ) );
+                    st.pix[ k ] = make_int2( o.pix, o.cpix );
                 }
                 if constexpr( MODE == 3 )
-                    if( task >= 0 )
+                    if( ended )
                     {   // for the adjoint: attenuation, segments inside the cut
                         P.adj_att[ task ] = att;
                         P.pq[ task ].cpix = ptau > P.tau_cut ? pk - 1 : pk;
                     }
-                const unsigned m_dep = __ballot_sync( m_fetch, dep );
-                if( ( int ) lane == leader && m_dep )
+                const int n_dep4 = 4 * __popc( m_dep );
+                __syncwarp(  );
+                for( int k = lane; k < n_dep4; k += 32 )
+                {
+                    const float v = reinterpret_cast< const float * >( st.v )[ k ];
+                    const int2  o = st.pix[ k >> 2 ];
+                    if( v != 0.0f )                   // V of light that was never circular
+                    {
+                        add_tally< TALLY >( P.image, P.c_image, ( size_t ) o.x * 4 + ( k & 3 ), v,
+                                            P.fx_scale );
+                        add_tally< TALLY >( P.img_batch, P.c_img_batch, ( size_t ) o.y * 4 + ( k & 3 ), v,
+                                            P.fx_scale );
+                    }
+                }
+                __syncwarp(  );
+                if( lane == 0 && m_dep )
                     atomicAdd( cnt_s + KP_CNT_DEPOSITS, ( unsigned long long ) __popc( m_dep ) );
             }
+            if( phase != PH_EMIT ) continue;
+            n_seg_done += pk;
             if constexpr( MODE == 1 )
                 if( task >= 0 )
                 {   // score of the ray that just ended (k_adjoint's measure ray)
