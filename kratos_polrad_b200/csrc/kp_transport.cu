@@ -38,7 +38,10 @@ namespace cg = cooperative_groups;
 // random numbers, so each packet's history equals a sequential walk that
 // marches every peel-off ray at the moment of its interaction.
 #ifndef KP_PEEL_BATCH
-#define KP_PEEL_BATCH 24             // k_peel: lanes that wait for a fetch batch
+#define KP_PEEL_BATCH 12             // k_peel: lanes that wait for a fetch batch (with
+                                     // the staged deposits: 24 -> 3.74, 16 -> 3.58,
+                                     // 12 -> 3.34, 8 -> 3.43 ms per 1e6 packets along x;
+                                     // obliquely 3.69, 3.55, 3.38, 3.30 ms per 3e5)
 #endif
 #ifndef KP_HOP_BATCH
 #define KP_HOP_BATCH 6               // lanes that wait for a batched block hand-off
@@ -47,11 +50,7 @@ namespace cg = cooperative_groups;
 #define KP_EMIT_BATCH 0              // lanes that wait for an emission batch (0: the event batch)
 #endif
 #ifndef KP_PEEL_INNER
-#define KP_PEEL_INNER 16             // k_peel: segments per scheduling round
-#endif
-#ifndef KP_PEEL_INNER_ADJ
-#define KP_PEEL_INNER_ADJ 8          // ... in the adjoint's marches (modes 1, 2): 4
-                                     // and 16 are slower there
+#define KP_PEEL_INNER 8              // k_peel: segments per scheduling round
 #endif
 #ifndef KP_PEEL_MINB
 #define KP_PEEL_MINB 4               // k_peel: resident blocks of 256 the registers allow
@@ -1020,8 +1019,7 @@ k_peel( const __grid_constant__ fwd_params_t P )
         }
 
         if( phase != PH_SEGMENT ) continue;
-        const int stop = min( pk + ( MODE == 1 || MODE == 2 ? KP_PEEL_INNER_ADJ : KP_PEEL_INNER ),
-                              1 << 20 );
+        const int stop = min( pk + KP_PEEL_INNER, 1 << 20 );
         #pragma unroll 1
         do
         {
