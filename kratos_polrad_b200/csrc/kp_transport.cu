@@ -1001,7 +1001,7 @@ k_peel( const __grid_constant__ fwd_params_t P )
             double x[ 3 ];                            // the crossing point: the new x0
             oray_point( P, x0, tc, x );
             int c[ 3 ] = { f0 - ( up0 ? 1 : 0 ), f1 - ( up1 ? 1 : 0 ), f2 - ( up2 ? 1 : 0 ) };
-            const bool left = ! cross_face( P.m, b, c, x, hop_ax, comp( P.o, hop_ax ) > 0.0f, lost );
+            const bool left = ! hand_off( P.m, b, c, x, hop_ax, comp( P.o, hop_ax ) > 0.0f, lost );
             const unsigned m_moved = __ballot_sync( m_hop, ! left && b != b_old );
             if( lane == ( unsigned ) ( __ffs( m_hop ) - 1 ) && m_moved )
                 atomicAdd( cnt_s + KP_CNT_HOPS, ( unsigned long long ) __popc( m_moved ) );

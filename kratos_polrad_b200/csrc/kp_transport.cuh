@@ -319,54 +319,46 @@ __device__ __forceinline__ double exit_dist( const mesh_view_t & m, int b, const
     return t;
 }
 
-// Steps into the neighbouring cell across face `ax` (x already advanced on
-// the other axes).  Returns false when the packet leaves the domain
-// (physical boundary) or finds no neighbour (lost = true).
-__device__ __forceinline__ bool cross_face( const mesh_view_t & m, int & b, int c[ 3 ],
-                                            double x[ 3 ], int ax, bool pos, bool & lost )
+// Hands a ray over the block's face (ax, side pos), which its cell c touches,
+// to the neighbour (x already advanced on the other axes): the new block's
+// cell, x snapped to its face (which also wraps a periodic boundary).
+// Returns false when the packet leaves the domain (physical boundary; x ends
+// on the face) or finds no neighbour (lost = true).
+// A hand-off is a chain of two loads (neighbour and level, then the new
+// block's geometry) that a batch of lanes waits for.  The face's level
+// difference and the boundary bits are read as single bytes: the record
+// indexed by face went through local memory.  The transverse cells are one
+// conversion (rounding down) clamped as an integer.  Walk 1.92 -> 1.85 ms and
+// march 3.38 -> 3.29 ms for 3e5 packets of the clump; the large scene, with
+// more hand-offs, 12.15 -> 11.47 and 6.27 -> 5.89 ms per 2e6.
+__device__ __forceinline__ bool hand_off( const mesh_view_t & m, int & b, int c[ 3 ], double x[ 3 ],
+                                          int ax, bool pos, bool & lost )
 {
     lost = false;
-    // select, not c[ ax ]: a runtime index would move c[] to local memory
-    const int cax = ax == 0 ? c[ 0 ] : ( ax == 1 ? c[ 1 ] : c[ 2 ] );
-    int cn = cax + ( pos ? 1 : -1 );
-    const double * g = m.geo_d + 16 * ( size_t ) b;
-    if( cn >= 0 && cn < m.nc[ ax ] )
-    {
-        #pragma unroll
-        for( int a = 0; a < 3; ++ a )
-            if( a == ax )
-            {
-                c[ a ] = cn;
-                x[ a ] = __fma_rn( ( double ) ( pos ? cn : cn + 1 ), g[ 3 + a ], g[ a ] );
-            }
-        return true;
-    }
-    const int side = pos ? 1 : 0;
+    const int side = pos ? 1 : 0, face = 2 * ax + side;
     // the face's four neighbour slots (16-byte aligned: 24 ints per block),
     // loaded together with the meta record, not after it
-    const int4 q = reinterpret_cast< const int4 * >( m.nb + 24 * ( size_t ) b )[ ax * 2 + side ];
-    const blk_meta_t md = m.meta[ b ];
-    if( ( md.phybnd >> ( 2 * ax + side ) ) & 1 )
+    const int4 q = reinterpret_cast< const int4 * >( m.nb + 24 * ( size_t ) b )[ face ];
+    const blk_meta_t * md = m.meta + b;
+    const int d_lvl = reinterpret_cast< const signed char * >( md )[ face ];
+    const unsigned phybnd = md->phybnd;
+    if( ( phybnd >> face ) & 1u )
     {   // leaves the domain: the position ends on the boundary face
+        const double * g = m.geo_d + 16 * ( size_t ) b;
         #pragma unroll
         for( int a = 0; a < 3; ++ a )
             if( a == ax )
-                x[ a ] = __fma_rn( ( double ) ( pos ? cax + 1 : cax ), g[ 3 + a ], g[ a ] );
+                x[ a ] = __fma_rn( ( double ) ( pos ? c[ a ] + 1 : c[ a ] ), g[ 3 + a ], g[ a ] );
         return false;
     }
-    const int a1 = ax == 2 ? 0 : ax + 1;
-    const int a2 = ax == 0 ? 2 : ax - 1;
-    int ca1 = 0, ca2 = 0;
-    #pragma unroll
-    for( int a = 0; a < 3; ++ a ) { if( a == a1 ) ca1 = c[ a ]; if( a == a2 ) ca2 = c[ a ]; }
     int j0 = 0, j1 = 0;
-    if( md.d_lvl[ 2 * ax + side ] > 0 )
-    {
-        j0 = ca1 >= m.nc[ a1 ] / 2;
-        j1 = ca2 >= m.nc[ a2 ] / 2;
+    if( d_lvl > 0 )
+    {   // the neighbour is finer: its half of the face by the transverse cells
+        const int a1 = ax == 2 ? 0 : ax + 1, a2 = ax == 0 ? 2 : ax - 1;
+        j0 = ( ax == 0 ? c[ 1 ] : ax == 1 ? c[ 2 ] : c[ 0 ] ) >= m.nc[ a1 ] / 2;
+        j1 = ( ax == 0 ? c[ 2 ] : ax == 1 ? c[ 0 ] : c[ 1 ] ) >= m.nc[ a2 ] / 2;
     }
-    const int js = j0 * 2 + j1;
-    const int nid = js == 0 ? q.x : ( js == 1 ? q.y : ( js == 2 ? q.z : q.w ) );
+    const int nid = j0 ? ( j1 ? q.w : q.z ) : ( j1 ? q.y : q.x );
     if( nid < 0 || nid >= m.n_blocks )
     {
         lost = true;
@@ -377,18 +369,40 @@ __device__ __forceinline__ bool cross_face( const mesh_view_t & m, int & b, int 
     #pragma unroll
     for( int a = 0; a < 3; ++ a )
     {
+        const double h0 = h[ a ], hd = h[ 3 + a ];
+        const int f = __double2int_rd( __dmul_rn( __dsub_rn( x[ a ], h0 ), h[ 8 + a ] ) );
+        const int last = m.nc[ a ] - 1;
         if( a == ax )
         {
-            c[ a ] = pos ? 0 : m.nc[ a ] - 1;
-            x[ a ] = pos ? h[ a ] : __fma_rn( ( double ) m.nc[ a ], h[ 3 + a ], h[ a ] );
+            c[ a ] = pos ? 0 : last;
+            x[ a ] = pos ? h0 : __fma_rn( ( double ) m.nc[ a ], hd, h0 );
         }
         else
-        {
-            const double f = floor( __dmul_rn( __dsub_rn( x[ a ], h[ a ] ), h[ 8 + a ] ) );
-            int ci = f < 0.0 ? 0 : ( f > ( double ) ( m.nc[ a ] - 1 ) ? m.nc[ a ] - 1 : ( int ) f );
-            c[ a ] = ci;
-        }
+            c[ a ] = min( max( f, 0 ), last );
     }
+    return true;
+}
+
+// Steps into the neighbouring cell across face `ax` (x already advanced on
+// the other axes).  Returns false when the packet leaves the domain
+// (physical boundary) or finds no neighbour (lost = true).
+__device__ __forceinline__ bool cross_face( const mesh_view_t & m, int & b, int c[ 3 ],
+                                            double x[ 3 ], int ax, bool pos, bool & lost )
+{
+    // select, not c[ ax ]: a runtime index would move c[] to local memory
+    const int cax = ax == 0 ? c[ 0 ] : ( ax == 1 ? c[ 1 ] : c[ 2 ] );
+    const int cn = cax + ( pos ? 1 : -1 );
+    if( cn < 0 || cn >= m.nc[ ax ] )
+        return hand_off( m, b, c, x, ax, pos, lost );
+    lost = false;
+    const double * g = m.geo_d + 16 * ( size_t ) b;
+    #pragma unroll
+    for( int a = 0; a < 3; ++ a )
+        if( a == ax )
+        {
+            c[ a ] = cn;
+            x[ a ] = __fma_rn( ( double ) ( pos ? cn : cn + 1 ), g[ 3 + a ], g[ a ] );
+        }
     return true;
 }
 
