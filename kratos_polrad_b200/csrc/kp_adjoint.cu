@@ -728,7 +728,8 @@ __global__ void k_adj_score( const __grid_constant__ fwd_params_t P )
 }
 
 // Deferred adjoint: adds the private path-length tallies of the depositing
-// march into grad_len (integer sums: the same result in any order).
+// march into grad_len (integer sums: the same result in any order; doubles in
+// the float mode).
 template< int TALLY >
 __global__ void k_adj_reduce( const __grid_constant__ fwd_params_t P )
 {
@@ -745,10 +746,11 @@ __global__ void k_adj_reduce( const __grid_constant__ fwd_params_t P )
         }
         else
         {
-            const float * q = static_cast< const float * >( P.adj_priv );
-            float v = 0.0f;
-            for( int k = 0; k < P.adj_npriv; ++ k ) v = __fadd_rn( v, q[ k * n + i ] );
-            if( v != 0.0f ) static_cast< float * >( P.g_len )[ i ] += v;
+            const double * q = static_cast< const double * >( P.adj_priv );
+            double v = 0.0;
+            for( int k = 0; k < P.adj_npriv; ++ k ) v = __dadd_rn( v, q[ k * n + i ] );
+            float * g = static_cast< float * >( P.g_len ) + i;
+            if( v != 0.0 ) * g = ( float ) __dadd_rn( ( double ) * g, v );
         }
     }
 }
@@ -763,7 +765,7 @@ void adjoint_buffers( kp_mesh_t * mesh, fwd_params_t & P, long long n_pk )
     const long long cap = mesh->pq_cap;
     const long long n_cells = ( long long ) P.m.n_blocks * P.m.cpb;
     const int n_priv = KP_ADJ_PRIV;
-    const size_t priv_bytes = n_priv > 1 ? ( size_t ) n_priv * n_cells * 8 : 0;
+    const size_t priv_bytes = ( size_t ) n_priv * n_cells * 8;
     // 256 B of counters, the per-packet and per-task arrays, then the private
     // tallies (256-byte aligned)
     const size_t adj_bytes = ( 256 + ( size_t ) n_pk * ( sizeof( double ) + 3 * sizeof( int ) )
@@ -791,8 +793,8 @@ void adjoint_buffers( kp_mesh_t * mesh, fwd_params_t & P, long long n_pk )
     P.adj_flag = P.adj_head + n_pk;
     P.adj_list = P.adj_flag + n_pk;
     P.pq_link  = reinterpret_cast< peel_link_t * >( P.adj_list + n_pk );
-    P.adj_priv = n_priv > 1 ? static_cast< char * >( mesh->d_adj ) + adj_bytes : nullptr;
-    P.adj_npriv = n_priv > 1 ? n_priv : 0;
+    P.adj_priv = static_cast< char * >( mesh->d_adj ) + adj_bytes;
+    P.adj_npriv = n_priv;
     P.pq = static_cast< peel_task_t * >( mesh->d_pq );
     P.pq_cap = cap;
 }
@@ -849,16 +851,12 @@ void adjoint_second_half( kp::fwd_params_t & C, int tally_mode, cudaStream_t s )
     if( fx ) kp::k_adj_walk< KP_TALLY_FIXED, 1 ><<< gw, threads, 0, s >>>( C );
     else     kp::k_adj_walk< KP_TALLY_FLOAT, 1 ><<< gw, threads, 0, s >>>( C );
     KP_CUDA( cudaGetLastError(  ) );
-    if( C.adj_priv )
-        KP_CUDA( cudaMemsetAsync( C.adj_priv, 0, ( size_t ) C.adj_npriv * n_cells * ( fx ? 8 : 4 ), s ) );
+    KP_CUDA( cudaMemsetAsync( C.adj_priv, 0, ( size_t ) C.adj_npriv * n_cells * 8, s ) );
     kp::launch_peel_adjoint( C, tally_mode, 2, s );
-    if( C.adj_priv )
-    {
-        const unsigned gr = ( unsigned ) std::min< long long >( 4096, ( n_cells + 255 ) / 256 );
-        if( fx ) kp::k_adj_reduce< KP_TALLY_FIXED ><<< gr, 256, 0, s >>>( C );
-        else     kp::k_adj_reduce< KP_TALLY_FLOAT ><<< gr, 256, 0, s >>>( C );
-        KP_CUDA( cudaGetLastError(  ) );
-    }
+    const unsigned gr = ( unsigned ) std::min< long long >( 4096, ( n_cells + 255 ) / 256 );
+    if( fx ) kp::k_adj_reduce< KP_TALLY_FIXED ><<< gr, 256, 0, s >>>( C );
+    else     kp::k_adj_reduce< KP_TALLY_FLOAT ><<< gr, 256, 0, s >>>( C );
+    KP_CUDA( cudaGetLastError(  ) );
     // packets whose rays found the queue full: both replays inline
     KP_CUDA( cudaMemsetAsync( C.work, 0, sizeof( unsigned long long ), s ) );
     C.adj_quiet = 1;

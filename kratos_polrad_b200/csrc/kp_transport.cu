@@ -844,12 +844,12 @@ k_peel( const __grid_constant__ fwd_params_t P )
     int    n_dep = 0;                             // MODE 2: ... and its segments
     // MODE 2: every ray leaves toward the observer along the same corridor of
     // cells, so the blocks deposit into private copies (summed afterwards)
-    // rather than all into one tally
-    void * g_dep = P.g_len;
+    // rather than all into one tally: int64, or doubles in the float mode
+    // (the copies' float sums were the larger part of its rounding noise)
+    unsigned long long * g_dep = nullptr;
     if constexpr( MODE == 2 )
-        if( P.adj_priv )
-            g_dep = ( char * ) P.adj_priv + ( size_t ) ( blockIdx.x % P.adj_npriv )
-                    * ( ( size_t ) P.m.n_blocks * P.m.cpb ) * ( TALLY == KP_TALLY_FIXED ? 8 : 4 );
+        g_dep = static_cast< unsigned long long * >( P.adj_priv )
+              + ( size_t ) ( blockIdx.x % P.adj_npriv ) * ( ( size_t ) P.m.n_blocks * P.m.cpb );
     long long task = -1;
     unsigned n_seg_done = 0;
     int phase = PH_EMIT;
@@ -1035,8 +1035,12 @@ k_peel( const __grid_constant__ fwd_params_t P )
             if constexpr( MODE == 2 )
             {   // the measuring march counted the segments inside the cut:
                 // geometry only, no coefficients
-                add_grad< TALLY >( g_dep, ( size_t ) ( eb - P.m.ext ) + ci,
-                                   __dmul_rn( -( double ) pG, back ? 0.0 : dt ), P.g_scale );
+                const size_t i = ( size_t ) ( eb - P.m.ext ) + ci;
+                const double v = __dmul_rn( -( double ) pG, back ? 0.0 : dt );
+                if constexpr( TALLY == KP_TALLY_FIXED )
+                    add_grad< TALLY >( g_dep, i, v, P.g_scale );
+                else
+                    atomicAdd( reinterpret_cast< double * >( g_dep ) + i, v );
                 if( pk >= n_dep )
                 {
                     phase = PH_EMIT;
