@@ -309,8 +309,9 @@ typedef struct kp_transport_cfg
     int       max_scatter;     /* interactions per packet before it is ended   */
     long long max_steps;       /* segments per packet before it is ended       */
     long long n_record;        /* final-state records for the first n packets  */
-    int       lane_batch;      /* scheduling: lanes of a warp that wait for an
-                                  interaction or emission batch (0: default 6)  */
+    int       lane_batch;      /* scheduling: packets of a warp that wait for an
+                                  interaction batch (0: default 32; 6 in
+                                  kp_transport_forward_noalloc)                 */
     int       flux_fx_shift;   /* fixed point of the flux tally (kp_tallies_t::
                                   flux): round(value * 2^flux_fx_shift); 0 takes
                                   fx_shift.  A cell's sum must stay below
@@ -499,7 +500,7 @@ typedef struct kp_scene
 
 typedef struct kp_tune_result
 {
-    int       threads;         /* threads per block (128 or 256)               */
+    int       threads;         /* threads per block                            */
     int       lane_batch;      /* event batch (see kp_transport_cfg_t)         */
     int       grid_pct;        /* persistent grid, percent of resident blocks  */
     float     sample_ms;       /* time of the best candidate on the sample     */
@@ -525,8 +526,7 @@ int kp_batch_forward( kp_batch_t * batch, const kp_transport_cfg_t * cfg, void *
  * (non-default), later calls replay it. */
 int kp_batch_graph_launch( kp_batch_t * batch, const kp_transport_cfg_t * cfg, void * mu,
                            unsigned long long * counters, void * stream );
-/* Autotuner: times candidate launch shapes (threads per block, event batch,
- * grid fill) on `fraction` of every scene's packets, tallying into
+/* Autotuner: times candidate launch shapes (event batch, grid fill) on `fraction` of every scene's packets, tallying into
  * mu_scratch (same shape as mu), and keeps the fastest for later launches. */
 int kp_batch_autotune( kp_batch_t * batch, const kp_transport_cfg_t * cfg, double fraction,
                        void * mu_scratch, void * stream, kp_tune_result_t * result );

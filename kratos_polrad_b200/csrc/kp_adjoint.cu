@@ -410,281 +410,6 @@ k_adjoint( const __grid_constant__ fwd_params_t P )
         atomicAdd( P.counters + threadIdx.x, sp.cnt[ threadIdx.x ] );
 }
 
-// Deferred adjoint, the walks.  PASS 0 walks every packet of the launch and
-// queues the peel-off ray of each vertex (the emission of an isotropic point
-// source and every interaction, when its point projects into the image) as
-// a task, linked in vertex order per packet; a packet whose ray finds the
-// queue full is flagged and listed for k_adjoint.  k_peel (mode 1) then
-// measures each ray's score G, k_adj_fold sums them per packet.  PASS 1
-// replays the walks with R, the sum of the scores of the interactions still
-// ahead (adj_R0 at the start, minus each vertex's G after it), and deposits
-// -R * length along the walk and R / sigma_sca at interactions; k_peel
-// (mode 2) deposits along the rays.  Per packet this is k_adjoint's
-// arithmetic in k_adjoint's order, so the int64 gradients are the same.
-template< int TALLY, int PASS >
-__global__ void __launch_bounds__( FWD_THREADS, 3 )
-k_adj_walk( const __grid_constant__ fwd_params_t P )
-{
-    struct cnt_park_t { unsigned long long cnt[ KP_NCOUNTERS ]; };
-    __shared__ cnt_park_t sp;
-    __shared__ cold_park_t< FWD_THREADS > sc;
-    const unsigned FULL = 0xffffffffu;
-    const unsigned lane = threadIdx.x & 31u;
-    if( threadIdx.x < KP_NCOUNTERS ) sp.cnt[ threadIdx.x ] = 0;
-    __syncthreads(  );
-    counts32_t cnt;
-    packet_t p;
-    double fx[ 3 ];
-    int phase = PH_EMIT, hop_ax = 0;
-    int lp = 0;        // the packet's index in the launch
-    int link = -1;     // PASS 0: its last task (-1 none, -2 the queue overflowed);
-                       // PASS 1: its next task
-    double R = 0.0;    // PASS 1
-
-    // PASS 0: queues the ray of vertex kv (toward the observer, weight w,
-    // Stokes I, Q, U, V), the lanes together with one atomic.
-    auto queue_ray = [ & ]( int pix, float w, float I, float Q, float U, float V, int kv )
-    {
-        const unsigned m = __activemask(  );
-        const int leader = __ffs( m ) - 1;
-        unsigned long long base = 0;
-        if( ( int ) lane == leader )
-            base = atomicAdd( P.pq_count, ( unsigned long long ) __popc( m ) );
-        base = __shfl_sync( m, base, leader );
-        const unsigned long long k = base + __popc( m & ( ( 1u << lane ) - 1u ) );
-        if( k >= ( unsigned long long ) P.pq_cap )
-        {   // the whole packet goes to k_adjoint
-            link = -2;
-            P.adj_flag[ lp ] = 1;
-            P.adj_list[ atomicAdd( P.adj_list_n, 1ull ) ] = lp;
-            return;
-        }
-        store_task( P.pq, k, p.x, p.b, p.c, w, I, Q, U, V, pix, 0 );
-        P.pq_link[ k ] = peel_link_t { lp, kv, -1 };
-        if( link >= 0 ) P.pq_link[ link ].next = ( int ) k;
-        else P.adj_head[ lp ] = ( int ) k;
-        link = ( int ) k;
-    };
-
-    for( ;; )
-    {
-        const unsigned m_emit = __ballot_sync( FULL, phase == PH_EMIT );
-        const unsigned m_seg  = __ballot_sync( FULL, phase == PH_SEGMENT );
-        const unsigned m_ev   = __ballot_sync( FULL, phase == PH_EVENT );
-        const unsigned m_hop  = __ballot_sync( FULL, phase == PH_HOP );
-        if( ( m_emit | m_seg | m_ev | m_hop ) == 0u )
-            break;
-        const int n_seg = __popc( m_seg ), n_ev = __popc( m_ev ), n_emit = __popc( m_emit );
-        const int n_hop = __popc( m_hop );
-        int run;
-        if( n_ev > 0 && ( n_ev >= P.ev_batch || n_seg == 0 ) )
-            run = PH_EVENT;
-        else if( n_emit > 0 && ( n_emit >= P.ev_batch || n_seg == 0 ) )
-            run = PH_EMIT;
-        else if( n_hop > 0 && ( n_hop >= P.hop_batch || n_seg == 0 ) )
-            run = PH_HOP;
-        else
-            run = PH_SEGMENT;
-
-        if( run == PH_HOP )
-        {
-            if( phase != PH_HOP ) continue;
-            const int b_old = p.b;
-            bool lost;
-            const bool left = ! cross_face( P.m, p.b, p.c, p.x, hop_ax,
-                                            comp( p.d, hop_ax ) > 0.0f, lost );
-            if( left )
-            {
-                count( sp, lost ? KP_CNT_LOST : KP_CNT_ESCAPED );
-                phase = PH_EMIT;
-                continue;
-            }
-            faces_all( P.m, p.b, p.c, p.d, fx );
-            if( p.b != b_old ) count( sp, KP_CNT_HOPS );
-            if( p.n_steps >= P.max_steps )
-            {
-                count( sp, KP_CNT_CAPPED );
-                phase = PH_EMIT;
-            }
-            else
-                phase = PH_SEGMENT;
-            continue;
-        }
-
-        if( run == PH_EMIT )
-        {
-            if( phase != PH_EMIT ) continue;
-            const int leader = __ffs( m_emit ) - 1;
-            const unsigned rank = __popc( m_emit & ( ( 1u << lane ) - 1u ) );
-            unsigned long long base = 0;
-            if( ( int ) lane == leader )
-                base = atomicAdd( P.work, ( unsigned long long ) n_emit );
-            base = __shfl_sync( m_emit, base, leader );
-            const unsigned long long idx = base + rank;
-            if( idx >= ( unsigned long long ) P.n_packets )
-            {
-                phase = PH_DONE;
-                continue;
-            }
-            lp = ( int ) source_major( ( long long ) idx, P.n_packets, P.n_src );
-            if constexpr( PASS == 1 )
-                if( P.adj_flag[ lp ] )
-                    continue;                     // replayed by k_adjoint
-            const long long pid = P.pid0 + ( long long ) lp;
-            float peel_I;
-            if( ! emit_any( P, pid, p, peel_I ) )
-            {
-                atomicOr( P.m.status, ST_BAD_SOURCE );
-                continue;
-            }
-            if constexpr( PASS == 0 )
-            {
-                count( sp, KP_CNT_EMITTED );
-                link = -1;
-            }
-            else
-            {
-                link = P.adj_head[ lp ];
-                R = P.adj_R0[ lp ];
-            }
-            p.tau = sample_tau( p.rng );
-            store_cold( sc, p );
-            if( P.img_n > 0 && peel_I > 0.0f )
-            {   // direct light of the emission (unpolarized)
-                const int pix = image_pixel( P, p.x );
-                if( pix >= 0 )
-                {
-                    if constexpr( PASS == 0 )
-                        queue_ray( pix, p.w, peel_I, 0.0f, 0.0f, 0.0f, 0 );
-                    else if( link >= 0 )
-                        link = P.pq_link[ link ].next;     // its ray is deposited by k_peel
-                }
-            }
-            faces_all( P.m, p.b, p.c, p.d, fx );
-            phase = PH_SEGMENT;
-            continue;
-        }
-
-        if( run == PH_EVENT )
-        {
-            if( phase != PH_EVENT ) continue;
-            load_cold( sc, p, P.seed );
-            ++ p.n_scat;
-            count( sp, KP_CNT_SCATTER );
-            const size_t ci = cell_index( P.m, p.b, p.c );
-            {
-                const float2 sg = P.m.sigma[ ci ];
-                p.w = __fmul_rn( p.w, __fdiv_rn( sg.x, __fadd_rn( sg.x, sg.y ) ) );
-                if constexpr( PASS == 1 )
-                    if( R != 0.0 )
-                        add_grad< TALLY >( P.g_int, ci, __ddiv_rn( R, ( double ) sg.x ), P.g_scale );
-            }
-            if( P.img_n > 0 )
-            {
-                const int pix = image_pixel( P, p.x );
-                if( pix >= 0 )
-                {
-                    if constexpr( PASS == 0 )
-                    {
-                        if( link != -2 )
-                        {
-                            float Q, U, V;
-                            const float I = phys::peel_stokes( P.ph, p.d, p.e1, p.S, P.o, P.ev,
-                                                               P.eh, Q, U, V );
-                            queue_ray( pix, p.w, I, Q, U, V, p.n_scat );
-                        }
-                    }
-                    else if( link >= 0 )
-                    {   // this vertex's score leaves R once its ray is deposited
-                        const float G = P.adj_G[ link ];
-                        link = P.pq_link[ link ].next;
-                        if( G != 0.0f )
-                            R = __dsub_rn( R, ( double ) G );
-                    }
-                }
-            }
-            int end = 0;
-            if( p.n_scat >= P.max_scatter )
-                end = PK_SCATTER_CAP;
-            else if( p.w < P.w_min )
-            {   // Russian roulette
-                const phys::u4 r = p.rng.next(  );
-                if( phys::u01( r.x ) < P.rr_survive )
-                    p.w = __fdiv_rn( p.w, P.rr_survive );
-                else
-                    end = PK_ABSORBED;
-            }
-            if( ! end )
-            {
-                phys::scatter( P.ph, p.rng, p.d, p.e1, p.S );
-                set_inv( p );
-                p.tau = sample_tau( p.rng );
-            }
-            if( ! end && p.n_steps >= P.max_steps )
-                end = PK_STEP_CAP;
-            if( end )
-                phase = PH_EMIT;
-            else
-            {
-                store_cold( sc, p );
-                faces_all( P.m, p.b, p.c, p.d, fx );
-                phase = PH_SEGMENT;
-            }
-            continue;
-        }
-
-        // ---- PH_SEGMENT: walk segments, up to KP_WALK_INNER per round ----
-        if( phase != PH_SEGMENT ) continue;
-        #pragma unroll 1
-        for( int it = 0; it < KP_WALK_INNER; ++ it )
-        {
-            const size_t ci = cell_index( P.m, p.b, p.c );
-            const float ext = P.m.ext[ ci ];
-            int ax;
-            const double t = exit_cached( p.x, fx, p.d, p.inv, ax );
-            const float et = __fmul_rn( ext, ( float ) t );
-            ++ cnt.steps;
-            ++ p.n_steps;
-            if( et >= p.tau )
-            {
-                double ti = ( double ) __fdiv_rn( p.tau, ext );
-                ti = ti > t ? t : ti;
-                if constexpr( PASS == 1 )
-                    if( R != 0.0 )
-                        add_grad< TALLY >( P.g_len, ci, __dmul_rn( -R, ti ), P.g_scale );
-                p.x[ 0 ] = __fma_rn( ti, ( double ) p.d.x, p.x[ 0 ] );
-                p.x[ 1 ] = __fma_rn( ti, ( double ) p.d.y, p.x[ 1 ] );
-                p.x[ 2 ] = __fma_rn( ti, ( double ) p.d.z, p.x[ 2 ] );
-                phase = PH_EVENT;
-                break;
-            }
-            p.tau = __fsub_rn( p.tau, et );
-            if constexpr( PASS == 1 )
-                if( R != 0.0 )
-                    add_grad< TALLY >( P.g_len, ci, __dmul_rn( -R, t ), P.g_scale );
-            #pragma unroll
-            for( int a = 0; a < 3; ++ a )
-                if( a != ax ) p.x[ a ] = __fma_rn( t, ( double ) comp( p.d, a ), p.x[ a ] );
-            if( ! step_in_block( P.m, p.b, p.c, p.x, fx, ax, p.d ) )
-            {   // leaves the block: wait for a batched hand-off
-                hop_ax = ax;
-                phase = PH_HOP;
-                break;
-            }
-            if( p.n_steps >= P.max_steps )
-            {
-                count( sp, KP_CNT_CAPPED );
-                phase = PH_EMIT;
-                break;
-            }
-        }
-    }
-    count_all( sp, KP_CNT_STEPS, cnt.steps );
-    __syncthreads(  );
-    if( P.counters && threadIdx.x < KP_NCOUNTERS && sp.cnt[ threadIdx.x ] )
-        atomicAdd( P.counters + threadIdx.x, sp.cnt[ threadIdx.x ] );
-}
-
 // Deferred adjoint: R of each packet, the sum of its interactions' scores in
 // vertex order (k_adjoint's first replay).  Task indices grow along a
 // packet's list, which bounds the walk through it.
@@ -822,6 +547,7 @@ void adjoint_params( kp_mesh_t * mesh, const kp_transport_cfg_t * cfg, const flo
     kp_transport_cfg_t c = * cfg;
     c.n_record = 0;
     kp::make_fwd_params( mesh, c, none, P );
+    P.n_mu = 0;                             // the replays tally no escapes
     P.image = P.img_batch = P.mu_tally = nullptr;
     P.adj_img = reinterpret_cast< const float4 * >( adj_image );
     P.g_len = grad_len;
@@ -832,25 +558,20 @@ void adjoint_params( kp_mesh_t * mesh, const kp_transport_cfg_t * cfg, const flo
 // The adjoint once every queued ray of the chunk C has its score in adj_G:
 // R per packet, the second replay, the deposits along the rays, and the
 // packets left to k_adjoint (whose first replay counts nothing).
-void adjoint_second_half( kp::fwd_params_t & C, int tally_mode, cudaStream_t s )
+void adjoint_second_half( kp::fwd_params_t & C, kp::pool_mem_t & pool, int tally_mode, cudaStream_t s )
 {
     const bool fx = tally_mode == KP_TALLY_FIXED;
     const int threads = kp::FWD_THREADS;
     const long long n_cells = ( long long ) C.m.n_blocks * C.m.cpb;
-    const void * kw = fx ? ( const void * ) kp::k_adj_walk< KP_TALLY_FIXED, 1 >
-                         : ( const void * ) kp::k_adj_walk< KP_TALLY_FLOAT, 1 >;
     const void * ka = fx ? ( const void * ) kp::k_adjoint< KP_TALLY_FIXED >
                          : ( const void * ) kp::k_adjoint< KP_TALLY_FLOAT >;
     const long long blocks = ( C.n_packets + threads - 1 ) / threads;
-    const unsigned gw = ( unsigned ) std::min< long long >( kp::persistent_grid( kw, threads ), blocks );
     const unsigned ga = ( unsigned ) std::min< long long >( kp::persistent_grid( ka, threads ), blocks );
     const unsigned gf = ( unsigned ) std::min< long long >( 4096, ( C.n_packets + 255 ) / 256 );
     kp::k_adj_fold<<< gf, 256, 0, s >>>( C );                           // R per packet
     KP_CUDA( cudaGetLastError(  ) );
     KP_CUDA( cudaMemsetAsync( C.work, 0, sizeof( unsigned long long ), s ) );
-    if( fx ) kp::k_adj_walk< KP_TALLY_FIXED, 1 ><<< gw, threads, 0, s >>>( C );
-    else     kp::k_adj_walk< KP_TALLY_FLOAT, 1 ><<< gw, threads, 0, s >>>( C );
-    KP_CUDA( cudaGetLastError(  ) );
+    kp::launch_walk( C, pool, tally_mode, kp::WALK_ADJ1, s );
     KP_CUDA( cudaMemsetAsync( C.adj_priv, 0, ( size_t ) C.adj_npriv * n_cells * 8, s ) );
     kp::launch_peel_adjoint( C, tally_mode, 2, s );
     const unsigned gr = ( unsigned ) std::min< long long >( 4096, ( n_cells + 255 ) / 256 );
@@ -901,19 +622,15 @@ extern "C" int kp_transport_adjoint( kp_mesh_t * mesh, const kp_transport_cfg_t 
         if( P.n_packets == 0 ) return;
         auto s = ( cudaStream_t ) stream;
         mesh->refresh_ext( s );
-        const bool fx = cfg->tally_mode == KP_TALLY_FIXED;
-        const int threads = kp::FWD_THREADS;
         mesh->tape_id = 0;                  // the queue is overwritten
         // The vertices' peel-off rays go through the mesh's queue (12 rays per
         // packet, chunks of packets beyond that) and are marched by k_peel.
         kp::ensure_peel_queue( mesh, P.n_packets );
         const long long chunk = std::max< long long >( mesh->pq_cap / kp::PQ_PER_PACKET, 1 );
         kp::adjoint_buffers( mesh, P, std::min( chunk, P.n_packets ) );
+        kp::ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
         // both marches read the queue in the forward solve's order
         int * perm = kp::peel_sorted( mesh ) ? kp::ensure_task_sort( mesh, mesh->pq_cap ) : nullptr;
-        const void * kw0 = fx ? ( const void * ) kp::k_adj_walk< KP_TALLY_FIXED, 0 >
-                              : ( const void * ) kp::k_adj_walk< KP_TALLY_FLOAT, 0 >;
-        const long long grid_w = kp::persistent_grid( kw0, threads );
         static thread_local kp::fwd_params_t C;
         for( long long done = 0; done < P.n_packets; done += chunk )
         {
@@ -921,18 +638,14 @@ extern "C" int kp_transport_adjoint( kp_mesh_t * mesh, const kp_transport_cfg_t 
             C.pq_perm = perm;
             C.pid0 = P.pid0 + done;
             C.n_packets = std::min( chunk, P.n_packets - done );
-            const unsigned gw = ( unsigned ) std::min< long long >( grid_w,
-                                                                   ( C.n_packets + threads - 1 ) / threads );
             KP_CUDA( cudaMemsetAsync( C.work, 0, 4 * sizeof( unsigned long long ), s ) );
             KP_CUDA( cudaMemsetAsync( C.adj_head, 0xff, C.n_packets * sizeof( int ), s ) );
             KP_CUDA( cudaMemsetAsync( C.adj_flag, 0, C.n_packets * sizeof( int ), s ) );
             // first replay: walks, vertex rays queued
-            if( fx ) kp::k_adj_walk< KP_TALLY_FIXED, 0 ><<< gw, threads, 0, s >>>( C );
-            else     kp::k_adj_walk< KP_TALLY_FLOAT, 0 ><<< gw, threads, 0, s >>>( C );
-            KP_CUDA( cudaGetLastError(  ) );
+            kp::launch_walk( C, mesh->pool, cfg->tally_mode, kp::WALK_ADJ0, s );
             if( perm ) kp::task_sort( mesh, C, s );                     // by starting cell
             kp::launch_peel_adjoint( C, cfg->tally_mode, 1, s );       // scores G
-            adjoint_second_half( C, cfg->tally_mode, s );
+            adjoint_second_half( C, mesh->pool, cfg->tally_mode, s );
         }
     } );
 }
@@ -952,7 +665,6 @@ extern "C" int kp_transport_forward_tape( kp_mesh_t * mesh, const kp_transport_c
         kp::make_fwd_params( mesh, * cfg, * tallies, P );
         if( P.n_packets == 0 ) return;
         mesh->refresh_ext( ( cudaStream_t ) stream );
-        if( cfg->lane_batch == 0 ) P.ev_batch = 12;
         kp::ensure_peel_queue( mesh, P.n_packets );
         if( P.n_packets > std::max< long long >( mesh->pq_cap / kp::PQ_PER_PACKET, 1 ) )
         {   // more packets than one chunk of the queue: an untaped solve
@@ -962,6 +674,7 @@ extern "C" int kp_transport_forward_tape( kp_mesh_t * mesh, const kp_transport_c
             return;
         }
         kp::adjoint_buffers( mesh, P, P.n_packets );
+        kp::ensure_pool( mesh->pool, P.n_packets, ( cudaStream_t ) stream );
         // the march order; the gradient's depositing march reads the same
         // permutation, which lives as long as the tape (every solve that
         // overwrites the queue drops the tape)
@@ -1008,7 +721,7 @@ extern "C" int kp_transport_adjoint_tape( kp_mesh_t * mesh, long long tape_id,
         const unsigned gs = 4 * 148;
         kp::k_adj_score<<< gs, 256, 0, s >>>( P );                        // G from the tape
         KP_CUDA( cudaGetLastError(  ) );
-        adjoint_second_half( P, cfg->tally_mode, s );
+        adjoint_second_half( P, mesh->pool, cfg->tally_mode, s );
     } );
 }
 

@@ -11,7 +11,7 @@
 // escape tallies.  A scene's packets are therefore identical to those of a
 // single-scene solve with the same seed and stream id.  The launch (counter
 // reset + kernel) can be captured once into a CUDA graph and replayed, and an
-// autotuner picks the block size, the event batch and the grid fill.
+// autotuner picks the event batch and the grid fill.
 #include "kp_transport.cuh"
 
 #include <algorithm>
@@ -38,11 +38,12 @@ struct kp_batch
     float      * d_ext = nullptr;              // sca + abs per cell, from d_sigma
     unsigned   * d_status = nullptr;
     unsigned long long * d_work = nullptr;
+    kp::pool_mem_t pool;                       // packets of the walk in progress
     long long  * d_prefix = nullptr;
     long long  * d_prefix_trial = nullptr;      // autotuner sample
     kp::scene_dev_t * d_scenes = nullptr;
     // launch shape (autotuned)
-    int threads = 256, lane_batch = 6, grid_pct = 100;
+    int threads = 128, lane_batch = 32, grid_pct = 100;
     // CUDA graph of the last launch configuration
     cudaGraphExec_t gexec = nullptr;
     kp::fwd_params_t gparams {  };
@@ -54,7 +55,7 @@ struct kp_batch
         cudaFree( d_nb ); cudaFree( d_meta ); cudaFree( d_geo ); cudaFree( d_sigma );
         cudaFree( d_ext );
         cudaFree( d_status ); cudaFree( d_work ); cudaFree( d_prefix );
-        cudaFree( d_prefix_trial ); cudaFree( d_scenes );
+        cudaFree( d_prefix_trial ); cudaFree( d_scenes ); cudaFree( pool.d );
     }
 };
 
@@ -95,7 +96,13 @@ void make_batch_params( kp_batch_t * b, const kp_transport_cfg_t & c, void * mu,
     P.mu_scene_stride = ( long long ) c.n_batches * c.n_mu_bins * 4;
     P.n_src = 1;
     P.work = b->d_work;
-    if( b->lane_batch > 0 && c.lane_batch == 0 ) P.ev_batch = b->lane_batch;
+    if( c.lane_batch == 0 ) P.ev_pool = b->lane_batch;
+}
+
+void launch( kp_batch_t * b, kp::fwd_params_t & P, int tally_mode, cudaStream_t s )
+{
+    KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
+    kp::launch_walk( P, b->pool, tally_mode, kp::WALK_FORWARD, s, b->grid_pct );
 }
 
 }   // namespace
@@ -193,6 +200,7 @@ int kp_batch_create( int n_scenes, const kp_scene_t * sc, kp_batch_t ** out )
                              cudaMemcpyHostToDevice ) );
         KP_CUDA( cudaMemcpy( b->d_scenes, b->scenes.data(  ),
                              b->scenes.size(  ) * sizeof( kp::scene_dev_t ), cudaMemcpyHostToDevice ) );
+        kp::ensure_pool( b->pool, b->total, nullptr );
         copy_sigma( b.get(  ), nullptr );
         KP_CUDA( cudaDeviceSynchronize(  ) );
         auto & v = b->view;
@@ -245,7 +253,7 @@ int kp_batch_forward( kp_batch_t * b, const kp_transport_cfg_t * cfg, void * mu,
         require( b && cfg, "null argument" );
         static thread_local kp::fwd_params_t P;
         make_batch_params( b, * cfg, mu, counters, P, false );
-        kp::launch_forward( P, cfg->tally_mode, ( cudaStream_t ) stream, b->threads, b->grid_pct );
+        launch( b, P, cfg->tally_mode, ( cudaStream_t ) stream );
     } );
 }
 
@@ -267,7 +275,7 @@ int kp_batch_graph_launch( kp_batch_t * b, const kp_transport_cfg_t * cfg, void 
             KP_CUDA( cudaStreamBeginCapture( s, cudaStreamCaptureModeThreadLocal ) );
             try
             {
-                kp::launch_forward( P, cfg->tally_mode, s, b->threads, b->grid_pct );
+                launch( b, P, cfg->tally_mode, s );
             }
             catch( ... )
             {
@@ -310,9 +318,8 @@ int kp_batch_autotune( kp_batch_t * b, const kp_transport_cfg_t * cfg, double fr
         cudaEvent_t e0, e1;
         KP_CUDA( cudaEventCreate( & e0 ) );
         KP_CUDA( cudaEventCreate( & e1 ) );
-        const int shapes[ ][ 3 ] = { { 256, 6, 100 }, { 256, 4, 100 }, { 256, 8, 100 },
-                                     { 256, 12, 100 }, { 128, 6, 100 }, { 128, 8, 100 },
-                                     { 256, 6, 75 }, { 128, 4, 100 } };
+        const int shapes[ ][ 3 ] = { { 128, 32, 100 }, { 128, 24, 100 }, { 128, 16, 100 },
+                                     { 128, 32, 80 }, { 128, 24, 80 } };
         constexpr int n_shapes = ( int ) ( sizeof( shapes ) / sizeof( shapes[ 0 ] ) );
         float t_min[ n_shapes ];
         for( int i = 0; i < n_shapes; ++ i ) t_min[ i ] = 1e30f;
@@ -332,7 +339,7 @@ int kp_batch_autotune( kp_batch_t * b, const kp_transport_cfg_t * cfg, double fr
                     kp::fwd_params_t P;
                     make_batch_params( b, c, mu_scratch, nullptr, P, true );
                     KP_CUDA( cudaEventRecord( e0, s ) );
-                    kp::launch_forward( P, c.tally_mode, s, b->threads, b->grid_pct );
+                    launch( b, P, c.tally_mode, s );
                     KP_CUDA( cudaEventRecord( e1, s ) );
                     KP_CUDA( cudaEventSynchronize( e1 ) );
                     float ms = 0;

@@ -92,6 +92,13 @@ struct alignas( 16 ) blk_meta_t
 };
 static_assert( sizeof( blk_meta_t ) == 16, "meta record" );
 
+// Device memory of the walk's packet pools (kp_walk.cu).
+struct pool_mem_t
+{
+    void * d = nullptr;
+    size_t bytes = 0;
+};
+
 struct mesh_view_t
 {
     int n_blocks;
@@ -158,6 +165,7 @@ struct kp_mesh
     float      * d_vol_f = nullptr;  double * d_vol_d = nullptr;
 
     unsigned long long * d_work = nullptr;   // scratch: packet counters
+    kp::pool_mem_t pool;                     // packets of the walk in progress
 
     kp::mesh_view_t view(  ) const;
     unsigned long long * workspace(  ) { upload( false ); return d_work; }

@@ -267,40 +267,40 @@ __device__ __forceinline__ float hg_mu( float g, float xi )
 // HG proposes mu from HG and accepts with (1 + r12 Q') / (1 + pmax).
 // (cos phi, sin phi) come from a point uniform in the unit disk.  At most 64
 // proposals; the last one is kept if all are rejected.
-__device__ __forceinline__ void scatter( const phase_t & ph, rng_t & rng, v3 & d,
-                                         v3 & e1, stokes_t & S )
+// One proposal from the draw r: (mu, a, b), whether it is accepted.  A point
+// outside the unit disk is rejected and leaves (a, b) = (1, 0).
+__device__ __forceinline__ bool scatter_trial( const phase_t & ph, const u4 & r, float q, float u,
+                                               float & mu, float & a, float & b )
 {
-    float mu = 0.0f, a = 1.0f, b = 0.0f, r2 = 1.0f, c2 = 1.0f, s2 = 0.0f, qp = S.q;
-    for( int trial = 0; trial < 64; ++ trial )
+    mu = ph.kind == 0 ? usym( r.x ) : hg_mu( ph.g, u01( r.x ) );
+    a  = usym( r.y );
+    b  = usym( r.z );
+    const float r2 = __fadd_rn( __fmul_rn( a, a ), __fmul_rn( b, b ) );
+    if( r2 > 1.0f || r2 == 0.0f )
     {
-        const u4 r = rng.next(  );
-        mu = ph.kind == 0 ? usym( r.x ) : hg_mu( ph.g, u01( r.x ) );
-        a  = usym( r.y );
-        b  = usym( r.z );
-        r2 = __fadd_rn( __fmul_rn( a, a ), __fmul_rn( b, b ) );
-        if( r2 > 1.0f || r2 == 0.0f )
-        {
-            a = 1.0f; b = 0.0f; r2 = 1.0f;
-            continue;
-        }
-        double_angle( a, b, c2, s2 );
-        qp = __fadd_rn( __fmul_rn( S.q, c2 ), __fmul_rn( S.u, s2 ) );
-        const float mu2 = __fmul_rn( mu, mu );
-        if( ph.kind == 0 )
-        {
-            const float f = __fadd_rn( __fadd_rn( 1.0f, mu2 ),
-                                       __fmul_rn( __fsub_rn( mu2, 1.0f ), qp ) );
-            if( __fmul_rn( 2.0f, u01( r.w ) ) < f ) break;
-        }
-        else
-        {
-            const float r12 = __fmul_rn( -ph.pmax, __fdiv_rn( __fsub_rn( 1.0f, mu2 ),
-                                                              __fadd_rn( 1.0f, mu2 ) ) );
-            const float f = __fadd_rn( 1.0f, __fmul_rn( r12, qp ) );
-            if( __fmul_rn( u01( r.w ), __fadd_rn( 1.0f, ph.pmax ) ) < f ) break;
-        }
+        a = 1.0f; b = 0.0f;
+        return false;
     }
+    float c2, s2;
+    double_angle( a, b, c2, s2 );
+    const float qp = __fadd_rn( __fmul_rn( q, c2 ), __fmul_rn( u, s2 ) );
+    const float mu2 = __fmul_rn( mu, mu );
+    if( ph.kind == 0 )
+    {
+        const float f = __fadd_rn( __fadd_rn( 1.0f, mu2 ), __fmul_rn( __fsub_rn( mu2, 1.0f ), qp ) );
+        return __fmul_rn( 2.0f, u01( r.w ) ) < f;
+    }
+    const float r12 = __fmul_rn( -ph.pmax, __fdiv_rn( __fsub_rn( 1.0f, mu2 ), __fadd_rn( 1.0f, mu2 ) ) );
+    const float f = __fadd_rn( 1.0f, __fmul_rn( r12, qp ) );
+    return __fmul_rn( u01( r.w ), __fadd_rn( 1.0f, ph.pmax ) ) < f;
+}
+
+// The scattering by (mu, phi), phi the angle of (a, b), r2 = a^2 + b^2.
+__device__ __forceinline__ void scatter_apply( const phase_t & ph, float mu, float a, float b,
+                                               float r2, v3 & d, v3 & e1, stokes_t & S )
+{
     // Stokes: rotate into the scattering plane, apply the matrix, normalize.
+    float c2, s2;
     double_angle( a, b, c2, s2 );
     float q = S.q, u = S.u;
     rotate( q, u, c2, s2 );
@@ -326,6 +326,15 @@ __device__ __forceinline__ void scatter( const phase_t & ph, rng_t & rng, v3 & d
     en = normalize( lin2( en, 1.0f, dn, -dot( en, dn ) ) );
     d  = dn;
     e1 = en;
+}
+
+__device__ __forceinline__ void scatter( const phase_t & ph, rng_t & rng, v3 & d,
+                                         v3 & e1, stokes_t & S )
+{
+    float mu = 0.0f, a = 1.0f, b = 0.0f;
+    for( int trial = 0; trial < 64; ++ trial )
+        if( scatter_trial( ph, rng.next(  ), S.q, S.u, mu, a, b ) ) break;
+    scatter_apply( ph, mu, a, b, __fadd_rn( __fmul_rn( a, a ), __fmul_rn( b, b ) ), d, e1, S );
 }
 
 // Peel-off toward the observer direction o with image frame (ev, eh = ev x o):

@@ -1,14 +1,10 @@
-// Forward polarized transport: persistent kernel with packet regeneration.
+// Forward polarized transport: the peel-off march, the single-kernel walk and
+// the entry points of the solves.
 //
-// Replaces the reference's per-cycle generate + integrate launches
-// (modules/particle/evolve/generate_par.h:51-62 -> ker_gen, then
-// evolve/integrator.h:47-63 -> ker_itg running photon::cart_t::proc) by one
-// persistent launch: every thread walks one packet at a time, segment by
-// segment, and when its packet ends (escape, absorption) it takes the next
-// packet index from a global counter.  Lanes that need new packets in the
-// same iteration take them with one warp-aggregated atomic (the warp's
-// coalesced group ballots, its leader adds the group size), so the warp
-// stays full while packet lifetimes differ by orders of magnitude.
+// A solve is the walk of its packets (k_walk, kp_walk.cu), which queues their
+// peel-off rays, then the march of the queue (k_peel).  k_forward is the
+// walk of the solves that have no memory for k_walk's packets or that cannot
+// queue their rays: kp_transport_forward_noalloc and the decomposed rounds.
 #include "kp_transport.cuh"
 
 #include <cub/cub.cuh>
@@ -46,17 +42,11 @@ namespace cg = cooperative_groups;
 #ifndef KP_HOP_BATCH
 #define KP_HOP_BATCH 6               // lanes that wait for a batched block hand-off
 #endif
-#ifndef KP_EMIT_BATCH
-#define KP_EMIT_BATCH 0              // lanes that wait for an emission batch (0: the event batch)
-#endif
 #ifndef KP_PEEL_INNER
 #define KP_PEEL_INNER 8              // k_peel: segments per scheduling round
 #endif
 #ifndef KP_PEEL_MINB
 #define KP_PEEL_MINB 4               // k_peel: resident blocks of 256 the registers allow
-#endif
-#ifndef KP_FWD_RESIDENT
-#define KP_FWD_RESIDENT 768          // resident threads per SM the register budget targets
 #endif
 
 // DD: one round of a domain-decomposed solve.  Work items are, in order, the
@@ -64,35 +54,19 @@ namespace cg = cooperative_groups;
 // this rank's emissions; a ray handed off into a block of another rank is
 // written to that rank's out-queue instead of continuing.  Each packet's
 // arithmetic is that of the replicated solve.
-// DEFER: a peel-off ray is written to the task queue for k_peel (when it
-// has room) instead of being marched here; the walk continues at once.
-// TAPE (with DEFER): the rays are also linked per packet, in vertex order,
-// for the adjoint of this solve (kp_transport_adjoint_tape); a packet with a
-// ray that found the queue full is flagged and listed instead.
 // FLUX: every walk segment adds w * dl / volume to its cell's flux tally,
 // the path-length estimator of photon::cart_t::proc_phys
 // (modules/particle/radiation/photon.h:73-83) with the packet's weight as
 // its `proper`; w / volume of the walk's block waits in shared memory (set
 // at emission, interactions and block hand-offs), so a segment adds one
 // multiply and one atomic.
-// RESUME (not with DD or TAPE): work items are first the packets an earlier
-// call suspended (P.rs_in), then the call's new packets; a packet that has
-// walked P.rs_budget segments in this launch (and is below max_steps) is
-// written whole to P.rs_out and left for a later call instead of ending.
-// Its arithmetic is that of an uninterrupted walk: the face cache and the
-// inverse direction are rebuilt bit for bit from the stored state.
-template< int TALLY, int NT, bool DD = false, bool DEFER = false, bool TAPE = false,
-          bool FLUX = false, bool RESUME = false >
-__global__ void __launch_bounds__( NT, KP_FWD_RESIDENT / NT )
+template< int TALLY, bool DD = false, bool FLUX = false >
+__global__ void __launch_bounds__( FWD_THREADS, 3 )
 k_forward( const __grid_constant__ fwd_params_t P )
 {
-    static_assert( ! ( RESUME && ( DD || TAPE ) ), "RESUME runs without DD and TAPE" );
-    __shared__ park_t< NT > sp;
-    __shared__ dir_park_t< NT > sd;
-    __shared__ cold_park_t< NT > sc;
-    // RESUME: the lane's packet stops (suspends or, at max_steps, ends) when
-    // its n_steps reaches this
-    __shared__ int s_stop[ RESUME ? NT : 1 ];
+    __shared__ park_t<  > sp;
+    __shared__ dir_park_t< FWD_THREADS > sd;
+    __shared__ cold_park_t< FWD_THREADS > sc;
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     if( threadIdx.x < KP_NCOUNTERS ) sp.cnt[ threadIdx.x ] = 0;
@@ -105,53 +79,13 @@ k_forward( const __grid_constant__ fwd_params_t P )
     float ptau = 0;               // fx the distances to its cell's faces (oray_faces)
     double ptc = 0.0;             // ... and ptc the distance it has travelled
     int pk = 0, pend = 0;
-    int si = 0;                                   // scene of a batched launch
     int hop_ax = 0;                               // face axis of a pending hand-off
     bool solo = false;                            // DD: peel-off ray without a parked walk
-    int tlink = -1;                               // TAPE: the packet's last task (-2: flagged)
-
-    // DEFER: appends the peel-off ray of vertex kv prepared in sp/sd
-    // (starting at p's position) to the queue; false when the queue is full.
-    // The lanes that append together take their slots with one atomic.
-    auto defer_peel = [ & ]( int kv ) -> bool
-    {
-        const unsigned m = __activemask(  );
-        const int leader = __ffs( m ) - 1;
-        unsigned long long base = 0;
-        if( ( int ) lane == leader )
-            base = atomicAdd( P.pq_count, ( unsigned long long ) __popc( m ) );
-        base = __shfl_sync( m, base, leader );
-        const unsigned long long k = base + __popc( m & ( ( 1u << lane ) - 1u ) );
-        const int lp = TAPE ? ( int ) ( p.pid(  ) - P.pid0 ) : 0;
-        if( k >= ( unsigned long long ) P.pq_cap )
-        {
-            if constexpr( TAPE )
-                if( tlink != -2 )
-                {   // the adjoint replays this packet with its rays inline
-                    tlink = -2;
-                    P.adj_flag[ lp ] = 1;
-                    P.adj_list[ atomicAdd( P.adj_list_n, 1ull ) ] = lp;
-                }
-            return false;
-        }
-        const int t = threadIdx.x;
-        store_task( P.pq, k, p.x, p.b, p.c, sp.w[ t ], sp.I[ t ], sp.Q[ t ], sp.U[ t ], sp.V[ t ],
-                    sp.pix[ t ], sd.cpix[ t ] );
-        if constexpr( TAPE )
-        {
-            P.pq_link[ k ] = peel_link_t { lp, kv, -1 };
-            if( tlink >= 0 ) P.pq_link[ tlink ].next = ( int ) k;
-            else P.adj_head[ lp ] = ( int ) k;
-            tlink = ( int ) k;
-        }
-        return true;
-    };
 
     // A peel-off ray marched by this lane at once from the packet's position
-    // (its contribution is in sp / sd): every ray of the single-kernel walk,
-    // and the rays that find the queue full in the deferred one.  Only the
-    // decomposed rounds schedule their rays segment by segment with the walk
-    // (a ray may cross into another rank's block mid-way).
+    // (its contribution is in sp / sd).  Only the decomposed rounds schedule
+    // their rays segment by segment with the walk (a ray may cross into another
+    // rank's block mid-way).
     auto peel_now = [ & ](  )
     {
         unsigned segs = 0, hops = 0;
@@ -225,8 +159,7 @@ k_forward( const __grid_constant__ fwd_params_t P )
         }
     };
 
-    // A whole walk (dd_walk_t) becomes the lane's packet: one arriving from
-    // another rank (DD), or one an earlier call suspended (RESUME).
+    // A whole walk (dd_walk_t) arriving from another rank becomes the lane's packet.
     auto load_walk = [ & ]( const dd_walk_t & o )
     {
         const int t = threadIdx.x;
@@ -255,20 +188,8 @@ k_forward( const __grid_constant__ fwd_params_t P )
         o.k1 = p.rng.k1; o.pid_lo = p.rng.pid_lo; o.pid_hi = p.rng.pid_hi;
         o.draw = p.rng.draw; o.batch = sc.batch[ threadIdx.x ];
     };
-    // RESUME: the packet (cold state loaded) leaves this launch unfinished.
-    auto suspend = [ & ](  )
-    {
-        const unsigned long long k = atomicAdd( P.rs_count, 1ull );
-        if( k < ( unsigned long long ) P.rs_cap )
-            store_walk( P.rs_out[ k ] );
-        else
-            atomicOr( P.m.status, ST_QUEUE_FULL );
-        phase = PH_EMIT;
-    };
-
     // After the active ray crossed a face (or stopped): the end of a peel-off
-    // ray (deposit, walk resumes) or of the packet's walk (escape, step cap,
-    // or, RESUME, the end of this launch's step budget).
+    // ray (deposit, walk resumes) or of the packet's walk (escape, step cap).
     // Shared by the segment phase and the hand-off phase.
     auto after_crossing = [ & ]( bool peel_cut, bool left, bool lost )
     {
@@ -318,20 +239,13 @@ k_forward( const __grid_constant__ fwd_params_t P )
             else
             {
                 end = PK_ESCAPED;
-                if( tally_escape< TALLY >( P, ( char * ) P.mu_tally + ( size_t ) si * P.mu_scene_stride
-                                             * ( TALLY == KP_TALLY_FIXED ? 8 : 4 ), P.c_mu, p,
-                                             sc.batch[ threadIdx.x ] ) )
+                if( tally_escape< TALLY >( P, P.mu_tally, P.c_mu, p, sc.batch[ threadIdx.x ] ) )
                     count( sp, KP_CNT_DEPOSITS );
             }
         }
-        else if( p.n_steps >= ( RESUME ? ( long long ) s_stop[ threadIdx.x ] : P.max_steps ) )
+        else if( p.n_steps >= P.max_steps )
         {
             load_cold( sc, p, P.seed );
-            if( RESUME && p.n_steps < P.max_steps )
-            {
-                suspend(  );
-                return;
-            }
             end = PK_STEP_CAP;
         }
         if( end )
@@ -356,8 +270,7 @@ k_forward( const __grid_constant__ fwd_params_t P )
         int run;
         if( n_ev > 0 && ( n_ev >= P.ev_batch || n_seg == 0 ) )
             run = PH_EVENT;
-        else if( n_emit > 0 && ( n_emit >= ( P.emit_batch > 0 ? P.emit_batch : P.ev_batch )
-                                 || n_seg == 0 ) )
+        else if( n_emit > 0 && ( n_emit >= P.ev_batch || n_seg == 0 ) )
             run = PH_EMIT;
         else if( n_hop > 0 && ( n_hop >= P.hop_batch || n_seg == 0 ) )
             run = PH_HOP;
@@ -495,44 +408,14 @@ k_forward( const __grid_constant__ fwd_params_t P )
                           : ( int ) ( pid % P.dd_ranks ) != P.dd_rank )
                     continue;
             }
-            else
+            else if( idx >= ( unsigned long long ) P.n_packets )
             {
-                if constexpr( RESUME )
-                {
-                    if( idx < ( unsigned long long ) P.rs_n_in )
-                    {   // a packet suspended by an earlier call goes on
-                        load_walk( P.rs_in[ idx ] );
-                        s_stop[ threadIdx.x ] = ( int ) min( P.max_steps,
-                                                             ( long long ) p.n_steps + P.rs_budget );
-                        phase = PH_SEGMENT;
-                        continue;
-                    }
-                    idx -= ( unsigned long long ) P.rs_n_in;
-                }
-                if( idx >= ( unsigned long long ) P.n_packets )
-                {
-                    phase = PH_DONE;
-                    continue;
-                }
+                phase = PH_DONE;
+                continue;
             }
             bool ok;
             float peel_I = 0.0f;          // emission's intensity toward the observer
-            if( P.n_scenes > 0 )
-            {   // batched launch: scene of this packet index, then its local id
-                int lo = 0, hi = P.n_scenes;
-                while( hi - lo > 1 )
-                {
-                    const int mid = ( lo + hi ) >> 1;
-                    if( ( long long ) idx >= P.scene_prefix[ mid ] ) lo = mid; else hi = mid;
-                }
-                si = lo;
-                const long long pid = P.pid0 + ( ( long long ) idx - P.scene_prefix[ si ] );
-                const src_dev_t & s = P.scenes[ si ].src;
-                ok = emit_packet( P, pid, p, s, P.scenes[ si ].stream );
-                peel_I = s.kind == KP_SOURCE_POINT && s.emit == KP_EMIT_ISOTROPIC ? 0x1.45f306p-4f
-                                                                                  : 0.0f;
-            }
-            else if constexpr( DD )
+            if constexpr( DD )
                 ok = emit_any( P, P.pid0 + ( long long ) idx, p, peel_I );
             else
                 ok = emit_any( P, P.pid0 + source_major( ( long long ) idx, P.n_packets, P.n_src ),
@@ -543,7 +426,6 @@ k_forward( const __grid_constant__ fwd_params_t P )
                 continue;
             }
             count( sp, KP_CNT_EMITTED );
-            if constexpr( TAPE ) tlink = -1;     // a new packet: its list starts empty
             sc.batch[ threadIdx.x ] = ( int ) ( p.pid(  ) % P.n_batch );
             p.tau = sample_tau( p.rng );
             phase = PH_SEGMENT;
@@ -595,12 +477,7 @@ k_forward( const __grid_constant__ fwd_params_t P )
                     sp.Q[ t ] = sp.U[ t ] = sp.V[ t ] = 0.0f;
                     sp.pix[ t ] = pix;
                     sd.cpix[ t ] = coarse_pixel( P, pix, sc.batch[ t ] );
-                    if constexpr( DEFER )
-                    {
-                        if( ! defer_peel( 0 ) )
-                            peel_now(  );
-                    }
-                    else if constexpr( ! DD )
+                    if constexpr( ! DD )
                         peel_now(  );
                     else
                     {
@@ -617,8 +494,6 @@ k_forward( const __grid_constant__ fwd_params_t P )
                 faces_all( P.m, p.b, p.c, p.d, fx );
             store_cold( sc, p );
             set_wv( p.w, p.b );
-            if constexpr( RESUME )
-                s_stop[ threadIdx.x ] = ( int ) min( P.max_steps, ( long long ) P.rs_budget );
             continue;
         }
 
@@ -670,9 +545,8 @@ k_forward( const __grid_constant__ fwd_params_t P )
                 end = PK_STEP_CAP;
             if constexpr( ! DD )
                 if( do_peel )
-                {   // queued, or marched here: the walk goes on (or ends) now
-                    if( ! DEFER || ! defer_peel( p.n_scat ) )
-                        peel_now(  );
+                {   // marched here: the walk goes on (or ends) now
+                    peel_now(  );
                     do_peel = false;
                 }
             if( do_peel )
@@ -689,8 +563,6 @@ k_forward( const __grid_constant__ fwd_params_t P )
                 count( sp, end == PK_ABSORBED ? KP_CNT_ABSORBED : KP_CNT_CAPPED );
                 phase = PH_EMIT;
             }
-            else if( RESUME && p.n_steps >= s_stop[ threadIdx.x ] )
-                suspend(  );             // the budget ran out with this segment
             else
                 phase = PH_SEGMENT;
             if( phase == PH_SEGMENT )
@@ -780,7 +652,7 @@ k_forward( const __grid_constant__ fwd_params_t P )
         atomicAdd( P.counters + threadIdx.x, sp.cnt[ threadIdx.x ] );
 }
 
-// Marches the peel-off rays k_forward<..., DEFER> queued: each lane takes a
+// Marches the peel-off rays that k_walk queued: each lane takes a
 // task, walks it toward the observer segment by segment exactly as the
 // forward kernel's inline peel-off ray does (same face distances, hand-off,
 // tau cut, deposit), and takes the next.  Fetches (with the deposit of the
@@ -1242,13 +1114,14 @@ void fill_common_params( const kp_transport_cfg_t & c, const kp_tallies_t & t,
     P.rr_survive = c.rr_survive > 0 ? c.rr_survive : 0.1f;
     P.max_scatter = c.max_scatter;
     P.max_steps = std::min< long long >( c.max_steps, 0x7fffffff );
+    // lanes (k_walk: packets of a warp) that wait for an interaction batch
     P.ev_batch = c.lane_batch > 0 ? c.lane_batch : 6;
+    P.ev_pool = c.lane_batch > 0 ? c.lane_batch : 32;
     // Block hand-offs wait for a batch of lanes (6 measured best for the
     // deferred walk and the peel-off march, 8 for the single-kernel walk
     // before it): the neighbour lookup and the new block's geometry are
     // dependent loads, paid once per batch.
     P.hop_batch = KP_HOP_BATCH;
-    P.emit_batch = KP_EMIT_BATCH;
     P.peel_batch = KP_PEEL_BATCH;
     P.mu_tally = t.mu;
     P.image = t.image;
@@ -1374,41 +1247,27 @@ int persistent_grid( const void * kernel, int threads )
     return n_sm * std::max( per_sm, 1 );
 }
 
-template< int TALLY, int NT, bool FLUX, bool RESUME = false >
-void launch_forward_k( const fwd_params_t & P, cudaStream_t s, int grid_pct )
+template< int TALLY, bool FLUX >
+void launch_forward_k( const fwd_params_t & P, cudaStream_t s )
 {
-    const void * k = ( const void * ) k_forward< TALLY, NT, false, false, false, FLUX, RESUME >;
-    long long grid = persistent_grid( k, NT );
-    grid = std::max< long long >( 1, grid * grid_pct / 100 );
-    grid = std::min< long long >( grid, ( P.n_packets + P.rs_n_in + NT - 1 ) / NT );
+    const long long grid = std::min< long long >( persistent_grid( ( const void * ) k_forward< TALLY, false, FLUX >,
+                                                                   FWD_THREADS ),
+                                                  ( P.n_packets + FWD_THREADS - 1 ) / FWD_THREADS );
     KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
-    // whole warps only: the scheduler ballots over full warps
-    k_forward< TALLY, NT, false, false, false, FLUX, RESUME ><<< ( unsigned ) grid, NT, 0, s >>>( P );
+    k_forward< TALLY, false, FLUX ><<< ( unsigned ) grid, FWD_THREADS, 0, s >>>( P );
     KP_CUDA( cudaGetLastError(  ) );
 }
 
-template< int NT >
-void launch_forward_nt( const fwd_params_t & P, int tally_mode, cudaStream_t s, int grid_pct )
-{
-    const bool fl = P.flux != nullptr;
-    if( tally_mode == KP_TALLY_FIXED )
-        fl ? launch_forward_k< KP_TALLY_FIXED, NT, true  >( P, s, grid_pct )
-           : launch_forward_k< KP_TALLY_FIXED, NT, false >( P, s, grid_pct );
-    else
-        fl ? launch_forward_k< KP_TALLY_FLOAT, NT, true  >( P, s, grid_pct )
-           : launch_forward_k< KP_TALLY_FLOAT, NT, false >( P, s, grid_pct );
-}
-
-// Launches the forward kernel with `threads` per block (128 or 256) and a
-// persistent grid of grid_pct percent of the resident-block capacity.
-void launch_forward( const fwd_params_t & P, int tally_mode, cudaStream_t s, int threads,
-                     int grid_pct )
+// The single-kernel walk: persistent grid, whole warps only (the scheduler
+// ballots over full warps).
+void launch_forward( const fwd_params_t & P, int tally_mode, cudaStream_t s )
 {
     if( P.n_packets == 0 ) return;
-    if( threads == 128 )
-        launch_forward_nt< 128 >( P, tally_mode, s, grid_pct );
+    const bool fl = P.flux != nullptr;
+    if( tally_mode == KP_TALLY_FIXED )
+        fl ? launch_forward_k< KP_TALLY_FIXED, true >( P, s ) : launch_forward_k< KP_TALLY_FIXED, false >( P, s );
     else
-        launch_forward_nt< 256 >( P, tally_mode, s, grid_pct );
+        fl ? launch_forward_k< KP_TALLY_FLOAT, true >( P, s ) : launch_forward_k< KP_TALLY_FLOAT, false >( P, s );
 }
 
 }   // namespace kp
@@ -1418,9 +1277,9 @@ namespace kp
 // Event recorded between the two kernels of a solve (kp_transport_split_event).
 thread_local cudaEvent_t split_event = nullptr;
 
-// Solve with peel-off rays deferred: k_forward<..., DEFER> walks the packets
-// and queues their peel-off rays (marching them inline only if the queue is
-// full), then k_peel marches the queue.  The queue belongs to the mesh and
+// Solve with peel-off rays deferred: k_walk walks the packets and queues
+// their peel-off rays (marching them inline only if the queue is full), then
+// k_peel marches the queue.  The queue belongs to the mesh and
 // holds 12 rays per packet, at most the mesh's limit (default 2^27 rays,
 // 8.6 GB); larger solves run in chunks of packets (cap / 12 packets each,
 // walk then march), so the queue is sized for the chunk, not the solve.
@@ -1442,16 +1301,6 @@ void ensure_peel_queue( kp_mesh_t * mesh, long long n_packets )
         KP_CUDA( cudaMalloc( & mesh->d_pq, ( size_t ) want * sizeof( peel_task_t ) ) );
         mesh->pq_cap = want;
     }
-}
-
-template< int TALLY, bool TAPE, bool FLUX, bool RESUME >
-void launch_deferred_walk( const fwd_params_t & P, cudaStream_t s )
-{
-    const void * kf = ( const void * ) k_forward< TALLY, 256, false, true, TAPE, FLUX, RESUME >;
-    long long grid = persistent_grid( kf, 256 );
-    grid = std::min< long long >( grid, ( P.n_packets + P.rs_n_in + 255 ) / 256 );
-    k_forward< TALLY, 256, false, true, TAPE, FLUX, RESUME ><<< ( unsigned ) grid, 256, 0, s >>>( P );
-    KP_CUDA( cudaGetLastError(  ) );
 }
 
 // Whether the forward solve marches the mesh's queue sorted by starting
@@ -1535,23 +1384,19 @@ void launch_peel( const fwd_params_t & P, cudaStream_t s )
     else                launch_peel_k< TALLY, MODE, false >( P, s );
 }
 
-template< int TALLY, bool TAPE, bool RESUME >
-void launch_deferred_chunk( fwd_params_t & P, cudaStream_t s, const kp_mesh_t * mesh )
+template< int TALLY, bool TAPE >
+void launch_deferred_chunk( fwd_params_t & P, cudaStream_t s, kp_mesh_t * mesh )
 {
-    require( P.pq_perm == nullptr || mesh, "peel-off sort without its mesh" );
     P.pq_count = P.work + 1;
     P.pq_next = P.work + 2;
     KP_CUDA( cudaMemsetAsync( P.work, 0, 3 * sizeof( unsigned long long ), s ) );
-    if( P.flux ) launch_deferred_walk< TALLY, TAPE, true,  RESUME >( P, s );
-    else         launch_deferred_walk< TALLY, TAPE, false, RESUME >( P, s );
+    launch_walk( P, mesh->pool, TALLY, WALK_FORWARD, s );
     if( split_event ) KP_CUDA( cudaEventRecord( split_event, s ) );
     if( P.pq_perm ) task_sort( mesh, P, s );
     launch_peel< TALLY, TAPE ? 3 : 0 >( P, s );
 }
-template void launch_deferred_chunk< KP_TALLY_FIXED, true, false >( fwd_params_t &, cudaStream_t,
-                                                                     const kp_mesh_t * );
-template void launch_deferred_chunk< KP_TALLY_FLOAT, true, false >( fwd_params_t &, cudaStream_t,
-                                                                     const kp_mesh_t * );
+template void launch_deferred_chunk< KP_TALLY_FIXED, true >( fwd_params_t &, cudaStream_t, kp_mesh_t * );
+template void launch_deferred_chunk< KP_TALLY_FLOAT, true >( fwd_params_t &, cudaStream_t, kp_mesh_t * );
 
 // The deferred adjoint's marches of the queued vertex rays: mode 1 measures
 // their scores, mode 2 deposits along them (k_peel).
@@ -1569,6 +1414,7 @@ void launch_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s )
     mesh->tape_id = 0;                      // the queue is overwritten
     ensure_peel_queue( mesh, P.n_packets );
     const long long chunk = std::max< long long >( mesh->pq_cap / PQ_PER_PACKET, 1 );
+    ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
     int * perm = peel_sorted( mesh ) ? ensure_task_sort( mesh, mesh->pq_cap ) : nullptr;
     static thread_local fwd_params_t C;
     for( long long done = 0; done < P.n_packets; done += chunk )
@@ -1579,7 +1425,7 @@ void launch_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s )
         C.pq_perm = perm;
         C.pid0 = P.pid0 + done;
         C.n_packets = std::min( chunk, P.n_packets - done );
-        launch_deferred_chunk< TALLY, false, false >( C, s, mesh );
+        launch_deferred_chunk< TALLY, false >( C, s, mesh );
     }
 }
 
@@ -1603,9 +1449,7 @@ extern "C" int kp_transport_forward( kp_mesh_t * mesh, const kp_transport_cfg_t 
         kp::make_fwd_params( mesh, * cfg, * tallies, P );
         P.work = mesh->workspace(  );
         if( cfg->image_n > 0 && P.n_packets > 0 )
-        {   // peel-off rays through their own kernel; without them the walk
-            // kernel's interactions run best in batches of 12 lanes (measured)
-            if( cfg->lane_batch == 0 ) P.ev_batch = 12;
+        {   // peel-off rays through their own kernel
             if( cfg->tally_mode == KP_TALLY_FIXED )
                 kp::launch_deferred< KP_TALLY_FIXED >( mesh, P, ( cudaStream_t ) stream );
             else
@@ -1613,9 +1457,16 @@ extern "C" int kp_transport_forward( kp_mesh_t * mesh, const kp_transport_cfg_t 
         }
         else
         {
-            kp::launch_forward( P, cfg->tally_mode, ( cudaStream_t ) stream, 256, 100 );
-            if( kp::split_event )
-                KP_CUDA( cudaEventRecord( kp::split_event, ( cudaStream_t ) stream ) );
+            auto s = ( cudaStream_t ) stream;
+            kp::ensure_pool( mesh->pool, P.n_packets, s );
+            if( mesh->pool.bytes == 0 )             // captured before the mesh's first solve
+                kp::launch_forward( P, cfg->tally_mode, s );
+            else
+            {
+                KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
+                kp::launch_walk( P, mesh->pool, cfg->tally_mode, kp::WALK_FORWARD, s );
+            }
+            if( kp::split_event ) KP_CUDA( cudaEventRecord( kp::split_event, s ) );
         }
         kp::fold_carry( * cfg, * tallies, ( cudaStream_t ) stream );
     } );
@@ -1660,7 +1511,7 @@ extern "C" int kp_transport_split_event( void * event )
 }
 
 ////////////////////////////////////////////////////////////
-// Resumable solve: the step budget of one call (k_forward<..., RESUME>).
+// Resumable solve: the step budget of one call (k_walk<..., RESUME>).
 
 static_assert( sizeof( kp_packet_state_t ) == sizeof( kp::dd_walk_t ), "packet state size" );
 static_assert( offsetof( kp_packet_state_t, n_steps ) == offsetof( kp::dd_walk_t, n_steps )
@@ -1680,6 +1531,7 @@ void launch_resume_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStrea
     mesh->tape_id = 0;                      // the queue is overwritten
     ensure_peel_queue( mesh, items );
     const long long chunk = std::max< long long >( mesh->pq_cap / PQ_PER_PACKET, 1 );
+    ensure_pool( mesh->pool, std::min( chunk, items ), s );
     int * perm = peel_sorted( mesh ) ? ensure_task_sort( mesh, mesh->pq_cap ) : nullptr;
     static thread_local fwd_params_t C;
     for( long long lo = 0; lo < items; lo += chunk )
@@ -1694,7 +1546,7 @@ void launch_resume_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStrea
         const long long first = std::max( lo, n_in );   // first new packet's item
         C.pid0 = P.pid0 + ( first - n_in );
         C.n_packets = std::max< long long >( hi - first, 0 );
-        launch_deferred_chunk< TALLY, false, true >( C, s, mesh );
+        launch_deferred_chunk< TALLY, false >( C, s, mesh );
     }
 }
 }   // namespace kp
@@ -1732,19 +1584,17 @@ extern "C" int kp_transport_forward_resume( kp_mesh_t * mesh, const kp_transport
         cudaStream_t s = ( cudaStream_t ) stream;
         if( P.n_packets + P.rs_n_in > 0 )
         {
-            const bool fx = cfg->tally_mode == KP_TALLY_FIXED, fl = P.flux != nullptr;
+            const bool fx = cfg->tally_mode == KP_TALLY_FIXED;
             if( cfg->image_n > 0 )
-            {   // the deferred walk's interaction batch, as kp_transport_forward
-                if( cfg->lane_batch == 0 ) P.ev_batch = 12;
+            {
                 fx ? kp::launch_resume_deferred< KP_TALLY_FIXED >( mesh, P, s )
                    : kp::launch_resume_deferred< KP_TALLY_FLOAT >( mesh, P, s );
             }
             else
             {
-                if( fx ) fl ? kp::launch_forward_k< KP_TALLY_FIXED, 256, true,  true >( P, s, 100 )
-                            : kp::launch_forward_k< KP_TALLY_FIXED, 256, false, true >( P, s, 100 );
-                else     fl ? kp::launch_forward_k< KP_TALLY_FLOAT, 256, true,  true >( P, s, 100 )
-                            : kp::launch_forward_k< KP_TALLY_FLOAT, 256, false, true >( P, s, 100 );
+                kp::ensure_pool( mesh->pool, P.n_packets + P.rs_n_in, s );
+                KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
+                kp::launch_walk( P, mesh->pool, cfg->tally_mode, kp::WALK_FORWARD, s );
                 if( kp::split_event ) KP_CUDA( cudaEventRecord( kp::split_event, s ) );
             }
         }
@@ -1753,7 +1603,7 @@ extern "C" int kp_transport_forward_resume( kp_mesh_t * mesh, const kp_transport
 }
 
 ////////////////////////////////////////////////////////////
-// One round of a domain-decomposed solve (k_forward<..., DD = true>).
+// One round of a domain-decomposed solve (k_forward<..., DD>).
 
 static_assert( sizeof( kp::dd_walk_t ) == KP_DD_WALK_BYTES, "walk record size" );
 
@@ -1762,10 +1612,10 @@ namespace kp
 template< int TALLY, bool FLUX >
 void launch_dd( const fwd_params_t & P, long long items, cudaStream_t s )
 {
-    const void * k = ( const void * ) k_forward< TALLY, 256, true, false, false, FLUX >;
+    const void * k = ( const void * ) k_forward< TALLY, true, FLUX >;
     long long grid = persistent_grid( k, 256 );
     grid = std::min< long long >( grid, ( items + 255 ) / 256 );
-    k_forward< TALLY, 256, true, false, false, FLUX ><<< ( unsigned ) grid, 256, 0, s >>>( P );
+    k_forward< TALLY, true, FLUX ><<< ( unsigned ) grid, 256, 0, s >>>( P );
     KP_CUDA( cudaGetLastError(  ) );
 }
 }   // namespace kp
@@ -1881,7 +1731,7 @@ extern "C" int kp_transport_forward_noalloc( kp_mesh_t * mesh, const kp_transpor
         kp::make_fwd_params( mesh, * cfg, * tallies, P );
         P.work = static_cast< unsigned long long * >( kp::noalloc_scratch(  ) );
         mesh->refresh_ext( ( cudaStream_t ) stream );    // a kernel into mesh memory
-        kp::launch_forward( P, cfg->tally_mode, ( cudaStream_t ) stream, 256, 100 );
+        kp::launch_forward( P, cfg->tally_mode, ( cudaStream_t ) stream );
         if( kp::split_event ) KP_CUDA( cudaEventRecord( kp::split_event, ( cudaStream_t ) stream ) );
         kp::fold_carry( * cfg, * tallies, ( cudaStream_t ) stream );
     } );

@@ -39,16 +39,20 @@ struct scene_dev_t
     uint32_t  pad;
 };
 
-// Walk segments per scheduling round of k_forward (but its decomposed rounds)
-// and k_adj_walk: 3 (forward walk 58.5 -> 56.9 ms, gradient 252 -> 247 ms,
-// batched launch 154.6 -> 151.5 ms against 2); the walk with the flux tally
-// keeps 2 (119 against 134 ms with 3).
+// Walk segments per scheduling round of k_forward (but its decomposed rounds):
+// 3, with the flux tally 2.
 #ifndef KP_WALK_INNER
 #define KP_WALK_INNER 3
 #endif
 #ifndef KP_WALK_INNER_FLUX
 #define KP_WALK_INNER_FLUX 2
 #endif
+
+// Packets of a warp's pool (kp_walk.cu).
+#ifndef KP_WALK_POOL
+#define KP_WALK_POOL 128
+#endif
+struct pool_chunk_t;
 
 // Everything a transport launch reads, passed by value.
 struct fwd_params_t
@@ -76,7 +80,7 @@ struct fwd_params_t
     int         max_scatter;
     long long   max_steps;
     int         ev_batch;          // lanes that must wait for an event batch
-    int         emit_batch;        // lanes that must wait for an emission batch (0: ev_batch)
+    int         ev_pool;           // k_walk: packets that must wait for an event batch
     int         hop_batch;         // lanes that must wait for a hand-off batch
     int         peel_batch;        // k_peel: lanes that must wait for a fetch batch
     double      lk_inv[ 3 ];       // lookup cells per unit length
@@ -92,6 +96,8 @@ struct fwd_params_t
     // float tallies' rounding-error carries (kp_tallies_t::carry; null: none)
     float     * c_image, * c_img_batch, * c_mu, * c_flux;
     unsigned long long * work;     // scratch: next packet index
+    pool_chunk_t * pool;           // k_walk: room for pool_n packets per warp
+    int         pool_n;
     // adjoint only
     const float4 * adj_img;        // dL/d(image) [img_n * img_n] (I, Q, U, V)
     void      * g_len;             // path-length term per cell
@@ -1094,12 +1100,23 @@ int * ensure_task_sort( kp_mesh_t * mesh, long long pq_cap );
 void task_sort( const kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s );
 // The walk of one chunk, then the march of its queue (in P.pq_perm's order
 // when set, sorted first with the mesh's buffers).
-template< int TALLY, bool TAPE, bool RESUME = false >
-void launch_deferred_chunk( fwd_params_t & P, cudaStream_t s, const kp_mesh_t * mesh = nullptr );
+template< int TALLY, bool TAPE >
+void launch_deferred_chunk( fwd_params_t & P, cudaStream_t s, kp_mesh_t * mesh );
 // A forward solve with its peel-off rays queued for k_peel, in chunks (no tape).
 void launch_deferred_solve( kp_mesh_t * mesh, const fwd_params_t & P, int tally_mode,
                             cudaStream_t s );
-void launch_forward( const fwd_params_t & P, int tally_mode, cudaStream_t s, int threads,
-                     int grid_pct );
+void launch_forward( const fwd_params_t & P, int tally_mode, cudaStream_t s );
+// The walk of one launch (k_walk): its kernel by P's queue, links, flux and
+// resume fields.  P.work, its packet counter, is zeroed by the caller.
+enum walk_kind { WALK_FORWARD = 0, WALK_ADJ0 = 1, WALK_ADJ1 = 2 };
+struct walk_shape_t
+{
+    long long warps;
+    int       per_warp;            // pool packets of a warp
+};
+walk_shape_t walk_shape( long long items, long long warps, const pool_mem_t & mem );
+void ensure_pool( pool_mem_t & mem, long long items, cudaStream_t s );
+void launch_walk( fwd_params_t & P, pool_mem_t & mem, int tally_mode, walk_kind kind, cudaStream_t s,
+                  int grid_pct = 100 );
 
 }   // namespace kp
