@@ -895,6 +895,11 @@ k_peel( const __grid_constant__ fwd_params_t P )
         #pragma unroll 1
         do
         {
+            // the cell's extinction, used only once the step is done: its gather
+            // overlaps the geometry (used before it: 3e5 packets obliquely 3.28
+            // against 2.92 ms, the large scene 5.88 against 5.02, along x 3.36
+            // against 3.24; loaded a segment ahead: 3.11, 5.88 and 3.42)
+            const float ext = MODE != 2 ? eb[ ci ] : 0.0f;
             // oray_segment: the nearest face (the first axis wins ties)
             const bool q1 = ! XZ && tm[ 1 ] < tm[ 0 ];
             double tn = q1 ? tm[ 1 ] : tm[ 0 ];
@@ -914,15 +919,6 @@ k_peel( const __grid_constant__ fwd_params_t P )
                 else
                     atomicAdd( reinterpret_cast< double * >( g_dep ) + i, v );
                 if( pk >= n_dep )
-                {
-                    phase = PH_EMIT;
-                    break;
-                }
-            }
-            else
-            {
-                ptau = __fadd_rn( ptau, __fmul_rn( eb[ ci ], back ? 0.0f : ( float ) dt ) );
-                if( ptau > P.tau_cut )
                 {
                     phase = PH_EMIT;
                     break;
@@ -956,6 +952,15 @@ k_peel( const __grid_constant__ fwd_params_t P )
                 ci += in ? st0 : 0;
                 hop_ax = 0;
                 tm[ 0 ] = face_dist( 0, f0 );
+            }
+            if constexpr( MODE != 2 )
+            {
+                ptau = __fadd_rn( ptau, __fmul_rn( ext, back ? 0.0f : ( float ) dt ) );
+                if( ptau > P.tau_cut )
+                {
+                    phase = PH_EMIT;
+                    break;
+                }
             }
             if( ! in )
             {
