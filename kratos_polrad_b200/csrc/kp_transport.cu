@@ -683,7 +683,11 @@ k_forward( const __grid_constant__ fwd_params_t P )
 // stages its rays' contributions in shared memory and four lanes add the four
 // components of one ray, one 32-byte sector; zeros (V, where the light was
 // never circular) are not added.  Along x 5.84 -> 3.74 ms, with float tallies
-// and their carries (whose atomics return) 6.15 -> 1.99 ms.
+// and their carries (whose atomics return) 6.15 -> 1.99 ms.  Float tallies:
+// the rays of one pixel in a batch (the direct rays of a source, a batch of
+// births) are summed in double first; one rounding then takes the place of
+// as many, and the pixel of a source is off by less
+// (1e6 packets of one source: 1.1e-5 of its sum, now 2e-8; 7.16 -> 7.07 ms).
 template< int TALLY, int MODE, bool XZ >
 __global__ void __launch_bounds__( 256, MODE == 2 ? 3 : KP_PEEL_MINB )
 k_peel( const __grid_constant__ fwd_params_t P )
@@ -691,6 +695,11 @@ k_peel( const __grid_constant__ fwd_params_t P )
     __shared__ unsigned long long cnt_s[ KP_NCOUNTERS ];
     struct stage_t { float4 v[ 32 ]; int2 pix[ 32 ]; };
     __shared__ stage_t stage[ MODE == 0 || MODE == 3 ? 8 : 1 ];   // one per warp
+    // float tallies: the sums per image pixel of a warp's contributions, as
+    // a float and what that float rounds off, at the pixel's first ray
+    struct stage_sum_t { float4 hi[ 32 ], lo[ 32 ]; unsigned first; };
+    constexpr bool SUMS = TALLY == KP_TALLY_FLOAT && ( MODE == 0 || MODE == 3 );
+    __shared__ stage_sum_t stage_sum[ SUMS ? 8 : 1 ];
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     if( threadIdx.x < KP_NCOUNTERS ) cnt_s[ threadIdx.x ] = 0;
@@ -786,6 +795,34 @@ k_peel( const __grid_constant__ fwd_params_t P )
                     st.v[ k ] = make_float4( __fmul_rn( att, o.I ), __fmul_rn( att, o.Q ),
                                              __fmul_rn( att, o.U ), __fmul_rn( att, o.V ) );
                     st.pix[ k ] = make_int2( o.pix, o.cpix );
+                    if constexpr( SUMS )
+                    {
+                        unsigned same = __match_any_sync( m_dep, o.pix );
+                        const bool first = lane == ( unsigned ) __ffs( same ) - 1u;
+                        stage_sum_t & ss = stage_sum[ threadIdx.x >> 5 ];
+                        if( lane == ( unsigned ) __ffs( m_dep ) - 1u ) ss.first = 0u;
+                        __syncwarp( m_dep );
+                        if( first )
+                        {
+                            double a[ 4 ] = { 0.0, 0.0, 0.0, 0.0 };
+                            for( ; same; same &= same - 1u )
+                            {
+                                const float4 v = st.v[ __popc( m_dep & ( ( same & -same ) - 1u ) ) ];
+                                a[ 0 ] = __dadd_rn( a[ 0 ], ( double ) v.x );
+                                a[ 1 ] = __dadd_rn( a[ 1 ], ( double ) v.y );
+                                a[ 2 ] = __dadd_rn( a[ 2 ], ( double ) v.z );
+                                a[ 3 ] = __dadd_rn( a[ 3 ], ( double ) v.w );
+                            }
+                            const float4 h = make_float4( ( float ) a[ 0 ], ( float ) a[ 1 ],
+                                                          ( float ) a[ 2 ], ( float ) a[ 3 ] );
+                            ss.hi[ k ] = h;
+                            ss.lo[ k ] = make_float4( ( float ) __dsub_rn( a[ 0 ], ( double ) h.x ),
+                                                      ( float ) __dsub_rn( a[ 1 ], ( double ) h.y ),
+                                                      ( float ) __dsub_rn( a[ 2 ], ( double ) h.z ),
+                                                      ( float ) __dsub_rn( a[ 3 ], ( double ) h.w ) );
+                            atomicOr( & ss.first, 1u << k );
+                        }
+                    }
                 }
                 if constexpr( MODE == 3 )
                     if( ended )
@@ -799,10 +836,25 @@ k_peel( const __grid_constant__ fwd_params_t P )
                 {
                     const float v = reinterpret_cast< const float * >( st.v )[ k ];
                     const int2  o = st.pix[ k >> 2 ];
+                    if constexpr( SUMS )
+                    {
+                        const stage_sum_t & ss = stage_sum[ threadIdx.x >> 5 ];
+                        if( ss.first >> ( k >> 2 ) & 1u )
+                        {
+                            const float  h = reinterpret_cast< const float * >( ss.hi )[ k ];
+                            const float  l = reinterpret_cast< const float * >( ss.lo )[ k ];
+                            const size_t i = ( size_t ) o.x * 4 + ( k & 3 );
+                            if( h != 0.0f )
+                                atomic_add_carry( static_cast< float * >( P.image ), P.c_image, i, h );
+                            if( l != 0.0f && P.c_image != nullptr )
+                                atomicAdd( P.c_image + i, l );
+                        }
+                    }
                     if( v != 0.0f )                   // V of light that was never circular
                     {
-                        add_tally< TALLY >( P.image, P.c_image, ( size_t ) o.x * 4 + ( k & 3 ), v,
-                                            P.fx_scale );
+                        if constexpr( ! SUMS )
+                            add_tally< TALLY >( P.image, P.c_image, ( size_t ) o.x * 4 + ( k & 3 ),
+                                                v, P.fx_scale );
                         add_tally< TALLY >( P.img_batch, P.c_img_batch, ( size_t ) o.y * 4 + ( k & 3 ), v,
                                             P.fx_scale );
                     }

@@ -57,3 +57,22 @@ def test_march_circular_light(azimuth):
     b = ref["image"] * 2.0 ** -t.fx_shift
     n_dep = int(ref["counters"][9])
     assert (np.abs(a - b) <= 1e-6 * np.abs(b[..., :1]) + n_dep * 2.0 ** -(t.fx_shift + 1)).all()
+
+
+@pytest.mark.parametrize("inclination,azimuth", [(60.0, 0.0), (70.0, 200.0)])
+def test_march_float_source_pixel(inclination, azimuth):
+    """Float tallies at the pixel of a source, where a large share of all rays
+    ends: within the final rounding (2^-24) and the carry's own (batches of up
+    to 32 rays are one addition: below 2e-7 at this count) of the fixed-point
+    sums, plus those sums' rounding of half a unit per deposit."""
+    mesh, sig, t = case("amr_point")
+    t = dataclasses.replace(t, n_packets=100_001, n_record=0, inclination_deg=inclination,
+                            azimuth_deg=azimuth)
+    mesh.set_sigma(sig)
+    fx = forward(mesh, to_device(t))
+    fl = forward(mesh, to_device(dataclasses.replace(t, tally_mode=TALLY_FLOAT)))
+    torch.cuda.synchronize()
+    b = fx.image.cpu().numpy() * 2.0 ** -t.fx_shift
+    a = fl.image.cpu().numpy().astype(np.float64)
+    n_dep = int(fx.counters.cpu().numpy()[9])
+    assert (np.abs(a - b) <= 3e-7 * np.abs(b[..., :1]) + n_dep * 2.0 ** -(t.fx_shift + 1)).all()
