@@ -55,7 +55,7 @@ struct kp_batch
         cudaFree( d_nb ); cudaFree( d_meta ); cudaFree( d_geo ); cudaFree( d_sigma );
         cudaFree( d_ext );
         cudaFree( d_status ); cudaFree( d_work ); cudaFree( d_prefix );
-        cudaFree( d_prefix_trial ); cudaFree( d_scenes ); cudaFree( pool.d );
+        cudaFree( d_prefix_trial ); cudaFree( d_scenes );
     }
 };
 

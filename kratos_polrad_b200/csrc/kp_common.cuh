@@ -97,6 +97,21 @@ struct pool_mem_t
 {
     void * d = nullptr;
     size_t bytes = 0;
+    void * old = nullptr;                 // an outgrown pool that a captured launch uses
+    bool   captured = false, full = false;
+
+    pool_mem_t(  ) = default;
+    pool_mem_t( const pool_mem_t & ) = delete;
+    pool_mem_t & operator=( const pool_mem_t & ) = delete;
+    ~ pool_mem_t(  ) { release(  ); }
+    void release(  )
+    {
+        cudaFree( d );
+        cudaFree( old );
+        d = old = nullptr;
+        bytes = 0;
+        captured = full = false;
+    }
 };
 
 struct mesh_view_t

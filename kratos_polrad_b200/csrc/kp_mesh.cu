@@ -188,7 +188,7 @@ void kp_mesh::release(  )
     cudaFree( d_lookup ); d_lookup = nullptr;
     cudaFree( d_status ); d_status = nullptr;
     cudaFree( d_work );   d_work   = nullptr;
-    cudaFree( pool.d );   pool     = kp::pool_mem_t {  };
+    pool.release(  );
     cudaFree( d_pq );     d_pq     = nullptr; pq_cap = 0;
     cudaFree( d_sort_cnt );  d_sort_cnt  = nullptr;
     cudaFree( d_sort_off );  d_sort_off  = nullptr;

@@ -1516,13 +1516,8 @@ extern "C" int kp_transport_forward( kp_mesh_t * mesh, const kp_transport_cfg_t 
         {
             auto s = ( cudaStream_t ) stream;
             kp::ensure_pool( mesh->pool, P.n_packets, s );
-            if( mesh->pool.bytes == 0 )             // captured before the mesh's first solve
-                kp::launch_forward( P, cfg->tally_mode, s );
-            else
-            {
-                KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
-                kp::launch_walk( P, mesh->pool, cfg->tally_mode, kp::WALK_FORWARD, s );
-            }
+            KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
+            kp::launch_walk( P, mesh->pool, cfg->tally_mode, kp::WALK_FORWARD, s );
             if( kp::split_event ) KP_CUDA( cudaEventRecord( kp::split_event, s ) );
         }
         kp::fold_carry( * cfg, * tallies, ( cudaStream_t ) stream );

@@ -847,34 +847,71 @@ walk_shape_t walk_shape( long long items, long long warps, const pool_mem_t & me
     return walk_shape_t { warps, ( int ) per };
 }
 
-// Makes the pool large enough for a launch of `items` packets.  A stream
-// that is being captured cannot allocate: its launch takes the pool there is.
+// Makes the pool large enough for a launch of `items` packets, at once where
+// a stream is being captured too.  A captured launch keeps its pool's address:
+// from then on a pool that is outgrown is kept (`old`) until its owner goes,
+// and the next one has the full size (48 MB on 148 SMs), so there is at most
+// one of these.  Where the memory is short, a smaller pool does.
 void ensure_pool( pool_mem_t & mem, long long items, cudaStream_t s )
 {
     int dev = 0, n_sm = 0;
     KP_CUDA( cudaGetDevice( & dev ) );
     KP_CUDA( cudaDeviceGetAttribute( & n_sm, cudaDevAttrMultiProcessorCount, dev ) );
-    const long long warps = ( long long ) n_sm * KP_WALK_MINB * WALK_WARPS;
-    const long long per = pool_size( items, warps );
-    const long long used = ( std::min( warps, items ) + WALK_WARPS - 1 ) / WALK_WARPS * WALK_WARPS;
-    const size_t want = ( size_t ) used * ( ( per + 31 ) / 32 ) * sizeof( pool_chunk_t );
-    if( mem.bytes >= want ) return;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     KP_CUDA( cudaStreamIsCapturing( s, & st ) );
-    if( st != cudaStreamCaptureStatusNone ) return;
-    cudaFree( mem.d );
-    mem.d = nullptr;
-    mem.bytes = 0;
-    KP_CUDA( cudaMalloc( & mem.d, want ) );
-    mem.bytes = want;
+    const bool capturing = st != cudaStreamCaptureStatusNone;
+    const long long warps = ( long long ) n_sm * KP_WALK_MINB * WALK_WARPS;
+    auto bytes = [ & ]( long long n )
+    {
+        const long long used = ( std::min( warps, n ) + WALK_WARPS - 1 ) / WALK_WARPS * WALK_WARPS;
+        return ( size_t ) used * ( ( pool_size( n, warps ) + 31 ) / 32 ) * sizeof( pool_chunk_t );
+    };
+    size_t want = bytes( items );
+    if( mem.bytes < want && ! mem.full )
+    {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;     // for this thread's allocation
+        KP_CUDA( cudaThreadExchangeStreamCaptureMode( & mode ) );
+        void * d = nullptr;
+        const bool keep = mem.captured || ( capturing && mem.d );
+        if( ! keep )
+        {
+            cudaFree( mem.d );
+            mem.d = nullptr;
+            mem.bytes = 0;
+        }
+        else
+            want = bytes( warps * KP_WALK_POOL );
+        cudaError_t e = cudaMalloc( & d, want );
+        const size_t least = std::max( mem.bytes, WALK_WARPS * sizeof( pool_chunk_t ) );
+        while( e == cudaErrorMemoryAllocation && want / 2 > least )
+        {
+            cudaGetLastError(  );
+            want /= 2;
+            e = cudaMalloc( & d, want );
+        }
+        cudaThreadExchangeStreamCaptureMode( & mode );
+        if( e == cudaSuccess )
+        {
+            if( keep ) mem.old = mem.d;
+            mem.d = d;
+            mem.bytes = want;
+            mem.full = keep;
+        }
+        else if( mem.d )
+            cudaGetLastError(  );                 // the pool there is
+        else
+        {
+            cudaGetLastError(  );
+            KP_CUDA( e );
+        }
+    }
+    mem.captured = mem.captured || capturing;
 }
 
 void launch_walk( fwd_params_t & P, pool_mem_t & mem, int tally_mode, walk_kind kind, cudaStream_t s,
                   int pct )
 {
     if( P.n_packets + P.rs_n_in == 0 ) return;
-    require( mem.bytes > 0, "the walk's first launch allocates its packet "
-             "pool: make it before capturing the stream", KP_ERR_CUDA );
     if( tally_mode == KP_TALLY_FIXED ) launch_walk_t< KP_TALLY_FIXED >( P, mem, kind, s, pct );
     else                               launch_walk_t< KP_TALLY_FLOAT >( P, mem, kind, s, pct );
 }

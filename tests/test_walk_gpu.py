@@ -84,3 +84,25 @@ def test_captured_walk_uses_the_pool_there_is():
         forward(first, t, again)
     g2.replay()
     _equal(again, want)
+
+
+@pytest.mark.parametrize("limit", [dict(), dict(max_steps=40)])
+def test_captured_walk_survives_a_larger_solve(limit):
+    """A solve captured before the mesh's first one, replayed after a solve
+    that outgrew its pool, and captured again at the larger count."""
+    mesh, t, want = _pair("slab", n_packets=5_000, **limit)
+    big = dataclasses.replace(t, n_packets=700_001)
+    got = Tallies(t)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        forward(mesh, t, got)
+    want_big = forward(mesh, big)
+    g.replay()
+    _equal(got, want)
+    again = Tallies(big)
+    g2 = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g2):
+        forward(mesh, big, again)
+    forward(mesh, dataclasses.replace(big, n_packets=900_001))
+    g2.replay()
+    _equal(again, want_big)
