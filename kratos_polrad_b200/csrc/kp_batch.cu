@@ -272,6 +272,7 @@ int kp_batch_graph_launch( kp_batch_t * b, const kp_transport_cfg_t * cfg, void 
         {   // (re)capture: counter reset + persistent kernel
             if( b->gexec ) { cudaGraphExecDestroy( b->gexec ); b->gexec = nullptr; }
             cudaGraph_t g = nullptr;
+            b->gparams = P;                       // what a later call is compared with
             KP_CUDA( cudaStreamBeginCapture( s, cudaStreamCaptureModeThreadLocal ) );
             try
             {
@@ -287,7 +288,6 @@ int kp_batch_graph_launch( kp_batch_t * b, const kp_transport_cfg_t * cfg, void 
             const cudaError_t e = cudaGraphInstantiate( & b->gexec, g, 0 );
             cudaGraphDestroy( g );
             KP_CUDA( e );
-            b->gparams = P;
             b->g_tally_mode = cfg->tally_mode;
         }
         KP_CUDA( cudaGraphLaunch( b->gexec, s ) );
