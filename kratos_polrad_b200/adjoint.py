@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import ctypes
 import dataclasses
+import math
 
 import torch
 
@@ -88,10 +89,13 @@ class TransportImage(torch.autograd.Function):
         # a = g / max|g| (order one, so the fixed-point deposits keep their
         # precision) and the result is scaled back by max|g| / N.
         gmax = g_img.abs().max()
-        if not torch.isfinite(gmax) or gmax == 0:
+        a = (g_img / gmax).to(torch.float32)
+        f = gmax / cfg.n_packets
+        # the only wait, and what it does not decide is launched before it (a
+        # gradient of 40009 packets at 48^3: 1.52 -> 1.47 ms against two waits)
+        g = gmax.item()
+        if not math.isfinite(g) or g == 0:
             z = torch.zeros(mesh.n_cells, dtype=torch.float64, device=g_img.device)
             return z, z.clone(), None, None, None
-        g_sca, g_abs = gradients(mesh, cfg, (g_img / gmax).to(torch.float32), ctx.shift,
-                                 tape_id=tape_id)
-        f = gmax / cfg.n_packets
+        g_sca, g_abs = gradients(mesh, cfg, a, ctx.shift, tape_id=tape_id)
         return g_sca * f, g_abs * f, None, None, None
