@@ -36,8 +36,12 @@ namespace cg = cooperative_groups;
 #ifndef KP_PEEL_BATCH
 #define KP_PEEL_BATCH 12             // k_peel: lanes that wait for a fetch batch (with
                                      // the staged deposits: 24 -> 3.74, 16 -> 3.58,
-                                     // 12 -> 3.34, 8 -> 3.43 ms per 1e6 packets along x;
-                                     // obliquely 3.69, 3.55, 3.38, 3.30 ms per 3e5)
+                                     // 12 -> 3.34, 8 -> 3.43 ms per 1e6 packets along x)
+#endif
+#ifndef KP_PEEL_BATCH_Y
+#define KP_PEEL_BATCH_Y 8            // ... where rays cross all three axes and segments
+                                     // are dearer (12 -> 2.93, 8 -> 2.85 ms per 3e5
+                                     // packets, inclination 52.5, azimuth 25)
 #endif
 #ifndef KP_HOP_BATCH
 #define KP_HOP_BATCH 6               // lanes that wait for a batched block hand-off
@@ -768,7 +772,7 @@ k_peel( const __grid_constant__ fwd_params_t P )
             break;
         const int n_fetch = __popc( m_fetch ), n_seg = __popc( m_seg ), n_hop = __popc( m_hop );
         int run;
-        if( n_fetch > 0 && ( n_fetch >= P.peel_batch || n_seg == 0 ) )
+        if( n_fetch > 0 && ( n_fetch >= ( XZ ? KP_PEEL_BATCH : KP_PEEL_BATCH_Y ) || n_seg == 0 ) )
             run = PH_EMIT;
         else if( n_hop > 0 && ( n_hop >= P.hop_batch || n_seg == 0 ) )
             run = PH_HOP;
@@ -1179,7 +1183,6 @@ void fill_common_params( const kp_transport_cfg_t & c, const kp_tallies_t & t,
     // before it): the neighbour lookup and the new block's geometry are
     // dependent loads, paid once per batch.
     P.hop_batch = KP_HOP_BATCH;
-    P.peel_batch = KP_PEEL_BATCH;
     P.mu_tally = t.mu;
     P.image = t.image;
     P.img_batch = t.image_batch;

@@ -82,7 +82,6 @@ struct fwd_params_t
     int         ev_batch;          // lanes that must wait for an event batch
     int         ev_pool;           // k_walk: packets that must wait for an event batch
     int         hop_batch;         // lanes that must wait for a hand-off batch
-    int         peel_batch;        // k_peel: lanes that must wait for a fetch batch
     double      lk_inv[ 3 ];       // lookup cells per unit length
     void      * mu_tally;
     void      * image;
