@@ -17,7 +17,7 @@
 // ahead), +R / sigma_sca at interactions, and -G_k * length along each
 // peel-off ray, subtracting G_k from R after vertex k.
 // kp_transport_adjoint runs this in five launches per chunk of packets
-// (k_adj_walk pass 0, k_peel measuring, k_adj_fold, k_adj_walk pass 1,
+// (k_walk WALK_ADJ0, k_peel measuring, k_adj_fold, k_walk WALK_ADJ1,
 // k_peel depositing), the vertices' rays queued between them; k_adjoint
 // does both passes in one launch with the rays inline (G_k kept in a
 // 32-entry per-lane array, later vertices re-measured in pass 1) and takes
@@ -669,7 +669,9 @@ extern "C" int kp_transport_forward_tape( kp_mesh_t * mesh, const kp_transport_c
         if( P.n_packets > std::max< long long >( mesh->pq_cap / kp::PQ_PER_PACKET, 1 ) )
         {   // more packets than one chunk of the queue: an untaped solve
             P.work = mesh->workspace(  );
+            kp::begin_flux( mesh, * tallies, cfg->tally_mode, P, ( cudaStream_t ) stream );
             kp::launch_deferred_solve( mesh, P, cfg->tally_mode, ( cudaStream_t ) stream );
+            kp::fold_flux( P, ( cudaStream_t ) stream );
             kp::fold_carry( * cfg, * tallies, ( cudaStream_t ) stream );
             return;
         }
@@ -684,10 +686,12 @@ extern "C" int kp_transport_forward_tape( kp_mesh_t * mesh, const kp_transport_c
         KP_CUDA( cudaMemsetAsync( P.work, 0, 4 * sizeof( unsigned long long ), s ) );
         KP_CUDA( cudaMemsetAsync( P.adj_head, 0xff, P.n_packets * sizeof( int ), s ) );
         KP_CUDA( cudaMemsetAsync( P.adj_flag, 0, P.n_packets * sizeof( int ), s ) );
+        kp::begin_flux( mesh, * tallies, cfg->tally_mode, P, s );
         if( cfg->tally_mode == KP_TALLY_FIXED )
             kp::launch_deferred_chunk< KP_TALLY_FIXED, true >( P, s, mesh );
         else
             kp::launch_deferred_chunk< KP_TALLY_FLOAT, true >( P, s, mesh );
+        kp::fold_flux( P, s );
         kp::fold_carry( * cfg, * tallies, s );
         mesh->tape_cfg = * cfg;
         mesh->tape_cfg.sources = nullptr;

@@ -181,6 +181,7 @@ struct kp_mesh
 
     unsigned long long * d_work = nullptr;   // scratch: packet counters
     kp::pool_mem_t pool;                     // packets of the walk in progress
+    double     * d_flux = nullptr;           // a float solve's flux sums, one per cell
 
     kp::mesh_view_t view(  ) const;
     unsigned long long * workspace(  ) { upload( false ); return d_work; }

@@ -189,6 +189,7 @@ void kp_mesh::release(  )
     cudaFree( d_status ); d_status = nullptr;
     cudaFree( d_work );   d_work   = nullptr;
     pool.release(  );
+    cudaFree( d_flux );   d_flux   = nullptr;
     cudaFree( d_pq );     d_pq     = nullptr; pq_cap = 0;
     cudaFree( d_sort_cnt );  d_sort_cnt  = nullptr;
     cudaFree( d_sort_off );  d_sort_off  = nullptr;

@@ -95,6 +95,7 @@ struct fwd_params_t
     // float tallies' rounding-error carries (kp_tallies_t::carry; null: none)
     float     * c_image, * c_img_batch, * c_mu, * c_flux;
     unsigned long long * work;     // scratch: next packet index
+    double    * flux_sum;          // k_walk, float tallies: the flux in double (null: P.flux)
     pool_chunk_t * pool;           // k_walk: room for pool_n packets per warp
     int         pool_n;
     // adjoint only
@@ -1107,6 +1108,10 @@ void launch_deferred_solve( kp_mesh_t * mesh, const fwd_params_t & P, int tally_
 void launch_forward( const fwd_params_t & P, int tally_mode, cudaStream_t s );
 // The walk of one launch (k_walk): its kernel by P's queue, links, flux and
 // resume fields.  P.work, its packet counter, is zeroed by the caller.
+// Sums a float solve's flux in double, in the mesh's own array (P.flux_sum),
+// and adds the sums into the tally at its end.
+void begin_flux( kp_mesh_t * mesh, const kp_tallies_t & t, int tally_mode, fwd_params_t & P, cudaStream_t s );
+void fold_flux( const fwd_params_t & P, cudaStream_t s );
 enum walk_kind { WALK_FORWARD = 0, WALK_ADJ0 = 1, WALK_ADJ1 = 2 };
 struct walk_shape_t
 {

@@ -214,6 +214,13 @@ k_walk( const __grid_constant__ fwd_params_t P )
         p.w = o.w[ i ]; p.n_scat = o.n_scat[ i ];
         p.rng = phys::rng_t { P.seed, o.k1[ i ], o.pid_lo[ i ], o.pid_hi[ i ], o.draw[ i ] };
     };
+    auto add_flux = [ & ]( size_t ic, double v )
+    {
+        if( TALLY == KP_TALLY_FLOAT && P.flux_sum )
+            atomicAdd( P.flux_sum + ic, v );
+        else
+            add_grad< TALLY >( P.flux, P.c_flux, ic, v, P.flux_scale );
+    };
     // RESUME: the packet leaves this launch unfinished
     auto suspend = [ & ]( const packet_t & p, int batch )
     {
@@ -598,8 +605,7 @@ k_walk( const __grid_constant__ fwd_params_t P )
                             double ti = ( double ) __fdiv_rn( tau, ext );
                             ti = ti > t ? t : ti;
                             if constexpr( FLUX )
-                                add_grad< TALLY >( P.flux, P.c_flux, ( size_t ) ( eb - P.m.ext ) + ci,
-                                                   __dmul_rn( ti, wv ), P.flux_scale );
+                                add_flux( ( size_t ) ( eb - P.m.ext ) + ci, __dmul_rn( ti, wv ) );
                             if constexpr( ADJ )
                                 if( wv != 0.0 )
                                     add_grad< TALLY >( P.g_len, ( size_t ) ( eb - P.m.ext ) + ci,
@@ -612,8 +618,7 @@ k_walk( const __grid_constant__ fwd_params_t P )
                         }
                         tau = __fsub_rn( tau, et );
                         if constexpr( FLUX )
-                            add_grad< TALLY >( P.flux, P.c_flux, ( size_t ) ( eb - P.m.ext ) + ci,
-                                               __dmul_rn( t, wv ), P.flux_scale );
+                            add_flux( ( size_t ) ( eb - P.m.ext ) + ci, __dmul_rn( t, wv ) );
                         if constexpr( ADJ )
                             if( wv != 0.0 )
                                 add_grad< TALLY >( P.g_len, ( size_t ) ( eb - P.m.ext ) + ci,

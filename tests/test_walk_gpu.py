@@ -10,7 +10,7 @@ import pytest
 import torch
 
 from kratos_polrad_b200 import _lib
-from kratos_polrad_b200.transport import PHASE_HG_POL, Tallies, forward
+from kratos_polrad_b200.transport import PHASE_HG_POL, TALLY_FLOAT, Tallies, forward
 from test_zz_no_alloc import _noalloc
 from transport_cases import case
 
@@ -106,3 +106,24 @@ def test_captured_walk_survives_a_larger_solve(limit):
     forward(mesh, dataclasses.replace(big, n_packets=900_001))
     g2.replay()
     _equal(again, want_big)
+
+
+@pytest.mark.parametrize("name,n,calls", [("slab", 33, 1), ("amr_point", 50_001, 1), ("hg_multi", 20_000, 3)])
+def test_float_flux_is_rounded_once_per_solve(name, n, calls):
+    """Float flux with a carry is summed in double and rounded once per call:
+    within 2^-24 per call (and the sum of the calls before) of the fixed-point
+    sums, plus those sums' half a unit per segment."""
+    mesh, sig, t = case(name)
+    t = dataclasses.replace(t, n_record=0, n_packets=n, flux=True, flux_fx_shift=30)
+    mesh.set_sigma(sig)
+    fx = Tallies(t, n_cells=mesh.n_cells)
+    tf = dataclasses.replace(t, tally_mode=TALLY_FLOAT)
+    fl = Tallies(tf, n_cells=mesh.n_cells)
+    for k in range(calls):
+        forward(mesh, dataclasses.replace(t, packet_offset=k * n), fx)
+        forward(mesh, dataclasses.replace(tf, packet_offset=k * n), fl)
+    torch.cuda.synchronize()
+    want = fx.flux.double() * fx.flux_scale()
+    steps = fx.counts()["steps"]
+    assert want.max() > 0
+    assert ((fl.flux.double() - want).abs() <= calls * 2.0 ** -24 * want + steps * 2.0 ** -31).all()
