@@ -129,7 +129,8 @@ def measured_peak():
 def ncu_traffic(n_packets):
     """DRAM bytes (read + write) of the two launches of one solve, per kernel,
     from the committed ncu summary (profiles/k_forward_clump_traffic.txt),
-    when it was captured on this packet count, else None."""
+    when it was captured on this packet count, else None.  The summary's key
+    for the walk, k_walk, is k_forward."""
     p = os.path.join(ROOT, "profiles", "k_forward_clump_traffic.txt")
     try:
         kv = {}
@@ -1034,12 +1035,12 @@ def main():
     traffic = ncu_traffic(n_pk)
     roofline = {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                 "frac": ach / peak, "peak_source": peak_kind,
-                "kernel": "k_forward + k_peel (the two launches of one solve)",
+                "kernel": "k_walk + k_peel (the two launches of one solve)",
                 "traffic": sum(traffic.values()) if traffic else None,
                 "algorithmic_bytes": algorithmic_bytes(c_rank),
                 "kernel_ms": statistics.mean(kern_ms),
-                "kernels": {"k_forward": {"ms": walk_ms, "share": walk_ms / (walk_ms + peel_ms),
-                                          "traffic": traffic and traffic["k_forward"]},
+                "kernels": {"k_walk": {"ms": walk_ms, "share": walk_ms / (walk_ms + peel_ms),
+                                       "traffic": traffic and traffic["k_forward"]},
                             "k_peel": {"ms": peel_ms, "share": peel_ms / (walk_ms + peel_ms),
                                        "traffic": traffic and traffic["k_peel"]}}}
 
