@@ -460,8 +460,9 @@ int kp_mesh_peel_queue_limit( kp_mesh_t * mesh, long long max_rays );
  * per 1e8 rays, up to 10 ms when one cell starts most of them, as a point
  * source's does; 4 B per ray plus 8 B per cell of device memory), so that
  * a warp marches rays that cross nearly the same cells: this pays when the
- * extinction field (4 B per cell) does not stay in L2.  KP_PEEL_ORDER_AUTO
- * (the default): CELL when the field exceeds KP_PEEL_SORT_MIN_BYTES, else
+ * extinction field (4 B per cell) is large.  KP_PEEL_ORDER_AUTO (the default):
+ * CELL when the field exceeds KP_PEEL_SORT_MIN_BYTES, or exceeds
+ * KP_PEEL_SORT_MANY_BYTES and the solve has KP_PEEL_SORT_MANY packets, else
  * QUEUE.  Fixed-point tallies are the same bit for bit in either order;
  * float tallies agree within rounding.  Other values are refused
  * (KP_ERR_CONFIG).  No counterpart in the reference. */
@@ -469,6 +470,8 @@ int kp_mesh_peel_queue_limit( kp_mesh_t * mesh, long long max_rays );
 #define KP_PEEL_ORDER_QUEUE 0
 #define KP_PEEL_ORDER_CELL  1
 #define KP_PEEL_SORT_MIN_BYTES ( 32ll << 20 )
+#define KP_PEEL_SORT_MANY_BYTES ( 12ll << 20 )
+#define KP_PEEL_SORT_MANY 500000
 int kp_mesh_peel_order( kp_mesh_t * mesh, int order );
 
 /* Profiling hook.  With an image, kp_transport_forward runs two kernels:

@@ -1411,16 +1411,22 @@ void ensure_peel_queue( kp_mesh_t * mesh, long long n_packets )
     }
 }
 
-// Whether the forward solve marches the mesh's queue sorted by starting
-// cell (kp_mesh_peel_order).  Measured: the 2-level clump scene (9.3 MB of
-// extinction, in L2) march took 59 + 10 ms sorted against 52 ms; the
-// 3-level large scene (83 MB) forward solve took 1.96 against 2.15 s.
-bool peel_sorted( const kp_mesh_t * mesh )
+// Whether a solve of n packets marches the mesh's queue sorted by starting
+// cell (kp_mesh_peel_order).  What the order saves is the march's L1 misses;
+// what it costs are four launches over the rays and the cells.  Solves as
+// queued and sorted: 9.3 MB of extinction (2-level clump) 66.1 and 68.9 ms per
+// 1e7 packets along x, 10.8 and 10.5 per 1e6 at inclination 60; 16 MB, a
+// gradient of 1e6 packets, 24.9 and 22.5; 20 MB 13.5 and 12.9; 32 MB 15.4 and
+// 14.6, and 1e5 packets 2.57 and 2.52, which the sort's buffers, about 1 ms on a
+// mesh's first such solve, outweigh; 51 MB 18.1 and 16.8; 74 MB 20.3 and 18.8.
+bool peel_sorted( const kp_mesh_t * mesh, long long n )
 {
     if( mesh->peel_order != KP_PEEL_ORDER_AUTO )
         return mesh->peel_order == KP_PEEL_ORDER_CELL;
     const auto v = mesh->view(  );
-    return ( long long ) v.n_blocks * v.cpb * ( long long ) sizeof( float ) > KP_PEEL_SORT_MIN_BYTES;
+    const long long bytes = ( long long ) v.n_blocks * v.cpb * ( long long ) sizeof( float );
+    return bytes > KP_PEEL_SORT_MIN_BYTES
+        || ( bytes > KP_PEEL_SORT_MANY_BYTES && n >= KP_PEEL_SORT_MANY );
 }
 
 // Makes room on the mesh for sorting a queue of pq_cap tasks (a permutation
@@ -1523,7 +1529,7 @@ void launch_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s )
     ensure_peel_queue( mesh, P.n_packets );
     const long long chunk = std::max< long long >( mesh->pq_cap / PQ_PER_PACKET, 1 );
     ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
-    int * perm = peel_sorted( mesh ) ? ensure_task_sort( mesh, mesh->pq_cap ) : nullptr;
+    int * perm = peel_sorted( mesh, P.n_packets ) ? ensure_task_sort( mesh, mesh->pq_cap ) : nullptr;
     static thread_local fwd_params_t C;
     for( long long done = 0; done < P.n_packets; done += chunk )
     {
@@ -1637,7 +1643,7 @@ void launch_resume_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStrea
     ensure_peel_queue( mesh, items );
     const long long chunk = std::max< long long >( mesh->pq_cap / PQ_PER_PACKET, 1 );
     ensure_pool( mesh->pool, std::min( chunk, items ), s );
-    int * perm = peel_sorted( mesh ) ? ensure_task_sort( mesh, mesh->pq_cap ) : nullptr;
+    int * perm = peel_sorted( mesh, items ) ? ensure_task_sort( mesh, mesh->pq_cap ) : nullptr;
     static thread_local fwd_params_t C;
     for( long long lo = 0; lo < items; lo += chunk )
     {
