@@ -26,10 +26,11 @@
 // (6.9 ms: 72% of the L1's data pipe); the crossed axis by branches (6.1 ms;
 // by selects, below, 5.6 ms).  Warp pools, fields in chunks of 32 and the
 // interaction's packet read again for its second half: 4.2 ms, against 6.0 ms
-// for the walk before.  Measured with this and the walk before: the clump
-// 5.96 -> 4.15 ms per 1e6 packets, 1.85 -> 1.47 ms per 3e5, 0.56 -> 0.24 ms
-// per 2000; the atmosphere 11.5 -> 8.5 ms per 1e6, 2.57 -> 1.16 ms per 1117; the
-// large scene 11.5 -> 9.0 ms per 2e6; the adjoint's replay 4.49 -> 3.86 ms.
+// for the walk before.  With the extinction ahead (AHEAD, below), against the
+// walk before: the clump 5.96 -> 3.99 ms per 1e6 packets, 1.85 -> 1.44 ms per
+// 3e5, 0.56 -> 0.24 ms per 2000; the atmosphere 11.5 -> 8.5 ms per 1e6, 2.57 ->
+// 1.15 ms per 1117; the large scene 11.5 -> 8.0 ms per 2e6; the adjoint's replay
+// 4.49 -> 3.86 ms.
 #include "kp_transport.cuh"
 
 namespace kp
@@ -461,7 +462,7 @@ k_walk( const __grid_constant__ fwd_params_t P )
             auto store_flight = [ & ](  )
             {
                 pool_chunk_t & o = pool[ slot >> 5 ];
-            const int i = slot & 31;
+                const int i = slot & 31;
                 #pragma unroll
                 for( int a = 0; a < 3; ++ a ) { o.x[ a ][ i ] = x[ a ]; o.c[ a ][ i ] = c[ a ]; }
                 o.tau[ i ] = tau; o.n_left[ i ] = n_left; o.b[ i ] = b;
