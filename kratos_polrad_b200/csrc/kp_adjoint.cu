@@ -630,7 +630,7 @@ extern "C" int kp_transport_adjoint( kp_mesh_t * mesh, const kp_transport_cfg_t 
         kp::adjoint_buffers( mesh, P, std::min( chunk, P.n_packets ) );
         kp::ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
         // both marches read the queue in the forward solve's order
-        int * perm = kp::peel_sorted( mesh, P.n_packets ) ? kp::ensure_task_sort( mesh, mesh->pq_cap ) : nullptr;
+        int * perm = kp::march_order( mesh, P.n_packets, s );
         static thread_local kp::fwd_params_t C;
         for( long long done = 0; done < P.n_packets; done += chunk )
         {
@@ -680,8 +680,8 @@ extern "C" int kp_transport_forward_tape( kp_mesh_t * mesh, const kp_transport_c
         // the march order; the gradient's depositing march reads the same
         // permutation, which lives as long as the tape (every solve that
         // overwrites the queue drops the tape)
-        const bool sorted = kp::peel_sorted( mesh, P.n_packets );
-        P.pq_perm = sorted ? kp::ensure_task_sort( mesh, mesh->pq_cap ) : nullptr;
+        P.pq_perm = kp::march_order( mesh, P.n_packets, ( cudaStream_t ) stream );
+        const bool sorted = P.pq_perm != nullptr;
         auto s = ( cudaStream_t ) stream;
         KP_CUDA( cudaMemsetAsync( P.work, 0, 4 * sizeof( unsigned long long ), s ) );
         KP_CUDA( cudaMemsetAsync( P.adj_head, 0xff, P.n_packets * sizeof( int ), s ) );

@@ -1464,6 +1464,35 @@ int * ensure_task_sort( kp_mesh_t * mesh, long long pq_cap )
     return mesh->d_sort_perm;
 }
 
+// The permutation of a solve of n packets that marches sorted, null for one
+// that marches as queued: also where only the count asked for the sort and
+// its buffers cannot be had (no memory left, a stream being captured).
+int * march_order( kp_mesh_t * mesh, long long n, cudaStream_t s )
+{
+    if( ! peel_sorted( mesh, n ) )
+        return nullptr;
+    if( ! peel_sorted( mesh, 0 ) )
+    {
+        const auto v = mesh->view(  );
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        KP_CUDA( cudaStreamIsCapturing( s, & st ) );
+        if( st != cudaStreamCaptureStatusNone
+            && ( mesh->sort_cells < ( size_t ) v.n_blocks * v.cpb
+                 || mesh->sort_perm < ( size_t ) mesh->pq_cap + 32 ) )
+            return nullptr;
+        try
+        {
+            return ensure_task_sort( mesh, mesh->pq_cap );
+        }
+        catch( const error_t & )
+        {
+            cudaGetLastError(  );
+            return nullptr;
+        }
+    }
+    return ensure_task_sort( mesh, mesh->pq_cap );
+}
+
 // Sorts the queued tasks by starting cell into P.pq_perm (k_task_sort).
 void task_sort( const kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s )
 {
@@ -1529,7 +1558,7 @@ void launch_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s )
     ensure_peel_queue( mesh, P.n_packets );
     const long long chunk = std::max< long long >( mesh->pq_cap / PQ_PER_PACKET, 1 );
     ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
-    int * perm = peel_sorted( mesh, P.n_packets ) ? ensure_task_sort( mesh, mesh->pq_cap ) : nullptr;
+    int * perm = march_order( mesh, P.n_packets, s );
     static thread_local fwd_params_t C;
     for( long long done = 0; done < P.n_packets; done += chunk )
     {
@@ -1643,7 +1672,7 @@ void launch_resume_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStrea
     ensure_peel_queue( mesh, items );
     const long long chunk = std::max< long long >( mesh->pq_cap / PQ_PER_PACKET, 1 );
     ensure_pool( mesh->pool, std::min( chunk, items ), s );
-    int * perm = peel_sorted( mesh, items ) ? ensure_task_sort( mesh, mesh->pq_cap ) : nullptr;
+    int * perm = march_order( mesh, items, s );
     static thread_local fwd_params_t C;
     for( long long lo = 0; lo < items; lo += chunk )
     {

@@ -1092,11 +1092,10 @@ void ensure_peel_queue( kp_mesh_t * mesh, long long n_packets );
 // for chunks of n_pk packets), with their own counters: P.work is set to
 // them, so launches that use the mesh's workspace do not touch a tape.
 void adjoint_buffers( kp_mesh_t * mesh, fwd_params_t & P, long long n_pk );
-// The march order of the mesh's queue (kp_mesh_peel_order): whether to
-// sort it by starting cell, the sort's buffers (returns the permutation),
-// and the sort of the queue P describes into P.pq_perm.
-bool peel_sorted( const kp_mesh_t * mesh, long long n );
-int * ensure_task_sort( kp_mesh_t * mesh, long long pq_cap );
+// The march order of the mesh's queue (kp_mesh_peel_order): the permutation's
+// buffer where it is to be sorted by starting cell (null: as queued), and the
+// sort of the queue P describes into P.pq_perm.
+int * march_order( kp_mesh_t * mesh, long long n, cudaStream_t s );
 void task_sort( const kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s );
 // The walk of one chunk, then the march of its queue (in P.pq_perm's order
 // when set, sorted first with the mesh's buffers).
