@@ -76,3 +76,23 @@ def test_march_float_source_pixel(inclination, azimuth):
     a = fl.image.cpu().numpy().astype(np.float64)
     n_dep = int(fx.counters.cpu().numpy()[9])
     assert (np.abs(a - b) <= 3e-7 * np.abs(b[..., :1]) + n_dep * 2.0 ** -(t.fx_shift + 1)).all()
+
+
+@pytest.mark.parametrize("n", [499_999, 500_000])
+def test_march_order_by_packet_count(n):
+    """On a mesh of 12 to 32 MB of extinction the order is chosen by the packet
+    count: the same int64 tallies as marched as queued, on either side."""
+    from kratos_polrad_b200.mesh import Mesh, MeshConfig, PEEL_ORDER_QUEUE
+    mesh = Mesh(MeshConfig((0, 0, 0), (1, 1, 1), (160,) * 3, (16,) * 3, (False,) * 3))
+    sig = np.empty((mesh.n_cells, 2), np.float32)
+    sig[:, 0], sig[:, 1] = 3.0, 0.5
+    mesh.set_sigma(sig)
+    _, _, t = case("amr_point")
+    t = dataclasses.replace(t, n_packets=n, n_record=0, fx_shift=30)
+    got = forward(mesh, t)
+    mesh.set_peel_order(PEEL_ORDER_QUEUE)
+    want = forward(mesh, t)
+    torch.cuda.synchronize()
+    assert mesh.status() == 0 and want.image.abs().sum() > 0
+    assert torch.equal(got.image, want.image) and torch.equal(got.image_batch, want.image_batch)
+    assert torch.equal(got.counters, want.counters)
