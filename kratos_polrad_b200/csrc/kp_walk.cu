@@ -505,6 +505,7 @@ k_walk( const __grid_constant__ fwd_params_t P )
                         const unsigned m_back = __ballot_sync( FULL, back );
                         if( back ) L.ready[ __popc( m_back & below ) ] = ( unsigned short ) slot;
                         n_ready = __popc( m_back );
+                        __syncwarp(  );       // the lists and the pool, read by other lanes next
                         break;
                     }
                     const int take = min( n_ready, n_idle );
