@@ -721,6 +721,9 @@ extern "C" int kp_transport_adjoint_tape( kp_mesh_t * mesh, long long tape_id,
         kp::adjoint_buffers( mesh, P, mesh->tape_n );      // the taped solve's layout
         P.pq_perm = mesh->tape_sorted ? mesh->d_sort_perm : nullptr;   // ... and order
         auto s = ( cudaStream_t ) stream;
+        // a solve without an image since then leaves the tape, but may have
+        // lost the pool for want of memory
+        kp::ensure_pool( mesh->pool, mesh->tape_n, s );
         mesh->refresh_ext( s );
         const unsigned gs = 4 * 148;
         kp::k_adj_score<<< gs, 256, 0, s >>>( P );                        // G from the tape

@@ -840,11 +840,13 @@ long long pool_size( long long items, long long warps )
 }
 
 // The warp count and pool size of a launch of `items` packets on a GPU that
-// holds `warps` warps, within the memory there is (at least a chunk for each
-// warp of a block).
+// holds `warps` warps, within the memory there is: at least a chunk for each
+// warp of a block, or the launch is refused (a warp without a pool would end
+// at once, and its packets with it).
 walk_shape_t walk_shape( long long items, long long warps, const pool_mem_t & mem )
 {
     const long long room = ( long long ) ( mem.bytes / sizeof( pool_chunk_t ) );    // chunks
+    require( room >= WALK_WARPS, "no pool for the walk's packets", KP_ERR_ALLOC );
     long long per = pool_size( items, warps );
     warps = std::min( std::min( warps, ( items + per - 1 ) / per ),
                       room / ( ( per + 31 ) / 32 ) / WALK_WARPS * WALK_WARPS );

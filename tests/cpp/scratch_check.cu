@@ -1,0 +1,216 @@
+// The library's host code against a CUDA runtime that only keeps books: every
+// allocation, free and launch of an entry point, without a GPU.  Linked with
+// the library's own objects in place of libcudart (tests/test_scratch.py).
+// Allocations get addresses that are never used twice, a limit on their sum
+// stands for the device's memory, and a stream (or another thread) can be
+// declared to be capturing.
+#include "kp_transport.cuh"
+
+#include <cstdio>
+#include <map>
+#include <set>
+#include <string>
+#include <vector>
+
+namespace
+{
+struct launch_t
+{
+    std::string kernel;
+    std::vector< void * > args;          // pointers among the arguments
+    kp::fwd_params_t P;                  // ... of a kernel that takes one
+};
+
+struct
+{
+    std::map< uintptr_t, size_t > live;
+    std::set< uintptr_t > freed;
+    std::map< const void *, std::string > names;
+    std::vector< launch_t > launches;
+    uintptr_t next = 1ull << 40;
+    size_t used = 0, limit = ~ ( size_t ) 0;
+    cudaStream_t capturing = nullptr;    // the stream that is being captured
+    bool other_captures = false;         // another thread captures, in the global mode
+    bool broken = false;                 // a call that such a capture does not survive
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
+    cudaError_t last = cudaSuccess;
+    long calls = 0;
+
+    bool unsafe(  )
+    {
+        const bool bad = mode != cudaStreamCaptureModeRelaxed && ( capturing || other_captures );
+        broken = broken || bad;
+        return bad;
+    }
+} F;
+
+cudaError_t ret( cudaError_t e )
+{
+    ++ F.calls;
+    if( e != cudaSuccess ) F.last = e;
+    return e;
+}
+
+int fails = 0;
+void expect( bool ok, const char * what )
+{
+    if( ! ok ) { std::printf( "FAIL %s\n", what ); ++ fails; }
+}
+}   // namespace
+
+void register_linked( void ( * cb )( void ** ), void *, void *, void ( * )( void * ) )
+{
+    static void * handle[ 2 ];
+    cb( handle );
+}
+
+#ifndef __CUDA_ARCH__                  // the device pass declares the runtime for kernels
+extern "C" {
+void fake_register( void ( * cb )( void ** ), void * a, void * b, void ( * c )( void * ) ) { register_linked( cb, a, b, c ); }
+void __cudaRegisterFunction( void **, const char * host, char *, const char * name, int, uint3 *, uint3 *, dim3 *, dim3 *, int * )
+{ F.names[ host ] = name; }
+void ** __cudaRegisterFatBinary( void * ) { static void * handle[ 2 ]; return handle; }
+void __cudaRegisterFatBinaryEnd( void ** ) {  }
+void __cudaUnregisterFatBinary( void ** ) {  }
+void __cudaRegisterVar( void **, char *, char *, const char *, int, size_t, int, int ) {  }
+static struct { dim3 g, b; size_t sh; cudaStream_t s; } conf;
+unsigned __cudaPushCallConfiguration( dim3 g, dim3 b, size_t sh, cudaStream_t s ) { conf = { g, b, sh, s }; return 0; }
+cudaError_t __cudaPopCallConfiguration( dim3 * g, dim3 * b, size_t * sh, void * s )
+{ * g = conf.g; * b = conf.b; * sh = conf.sh; * ( cudaStream_t * ) s = conf.s; return cudaSuccess; }
+cudaError_t cudaLaunchKernel( const void * f, dim3, dim3, void ** args, size_t, cudaStream_t )
+{
+    launch_t l {  };
+    l.kernel = F.names[ f ];
+    if( l.kernel.find( "12fwd_params_t" ) != std::string::npos )
+    {
+        std::memcpy( & l.P, args[ 0 ], sizeof( l.P ) );
+        if( l.kernel.find( "k_task_sort" ) != std::string::npos )
+            for( int k = 1; k < 3; ++ k ) l.args.push_back( * ( void ** ) args[ k ] );
+    }
+    F.launches.push_back( l );
+    return ret( cudaSuccess );
+}
+cudaError_t cudaMalloc( void ** p, size_t n )
+{
+    * p = nullptr;
+    if( F.unsafe(  ) ) return ret( cudaErrorStreamCaptureUnsupported );
+    if( F.used + n > F.limit ) return ret( cudaErrorMemoryAllocation );
+    * p = ( void * ) F.next;
+    F.live[ F.next ] = n;
+    F.used += n;
+    F.next += ( n + 4095 ) / 4096 * 4096 + 4096;
+    return ret( cudaSuccess );
+}
+cudaError_t cudaFree( void * p )
+{
+    if( p == nullptr ) return ret( cudaSuccess );
+    if( F.unsafe(  ) ) return ret( cudaErrorStreamCaptureUnsupported );
+    auto it = F.live.find( ( uintptr_t ) p );
+    expect( it != F.live.end(  ), "a free of what is not allocated" );
+    if( it == F.live.end(  ) ) return ret( cudaErrorInvalidValue );
+    F.used -= it->second;
+    F.freed.insert( it->first );
+    F.live.erase( it );
+    return ret( cudaSuccess );
+}
+cudaError_t cudaStreamIsCapturing( cudaStream_t s, cudaStreamCaptureStatus * st )
+{
+    * st = F.capturing && s == F.capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    return ret( cudaSuccess );
+}
+cudaError_t cudaThreadExchangeStreamCaptureMode( cudaStreamCaptureMode * m ) { std::swap( * m, F.mode ); return ret( cudaSuccess ); }
+cudaError_t cudaGetLastError( void ) { const auto e = F.last; F.last = cudaSuccess; ++ F.calls; return e; }
+cudaError_t cudaPeekAtLastError( void ) { return F.last; }
+const char * cudaGetErrorString( cudaError_t e ) { return e == cudaErrorMemoryAllocation ? "out of memory" : "error"; }
+cudaError_t cudaGetDevice( int * d ) { * d = 0; return ret( cudaSuccess ); }
+cudaError_t cudaSetDevice( int ) { return ret( cudaSuccess ); }
+cudaError_t cudaGetDeviceCount( int * n ) { * n = 1; return ret( cudaSuccess ); }
+cudaError_t cudaDeviceGetAttribute( int * v, cudaDeviceAttr, int ) { * v = 148; return ret( cudaSuccess ); }
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor( int * n, const void *, int, size_t ) { * n = 5; return ret( cudaSuccess ); }
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags( int * n, const void *, int, size_t, unsigned ) { * n = 5; return ret( cudaSuccess ); }
+cudaError_t cudaFuncGetAttributes( cudaFuncAttributes * a, const void * )
+{ * a = cudaFuncAttributes {  }; a->ptxVersion = a->binaryVersion = 100; return ret( cudaSuccess ); }
+cudaError_t cudaMemset( void *, int, size_t ) { return ret( cudaSuccess ); }
+cudaError_t cudaMemsetAsync( void *, int, size_t, cudaStream_t ) { return ret( cudaSuccess ); }
+cudaError_t cudaMemcpy( void *, const void *, size_t, cudaMemcpyKind ) { return ret( cudaSuccess ); }
+cudaError_t cudaMemcpyAsync( void *, const void *, size_t, cudaMemcpyKind, cudaStream_t ) { return ret( cudaSuccess ); }
+cudaError_t cudaDeviceSynchronize( void ) { return ret( cudaSuccess ); }
+cudaError_t cudaStreamSynchronize( cudaStream_t ) { return ret( cudaSuccess ); }
+}   // extern "C"
+#endif
+
+namespace
+{
+struct solve_t
+{
+    kp_transport_cfg_t cfg {  };
+    kp_tallies_t t {  };
+    kp_source_t src { KP_SOURCE_POINT, KP_EMIT_ISOTROPIC, { 0.5, 0.5, 0.5 } };
+    solve_t( long long n, bool image )
+    {
+        cfg.n_packets = n;
+        cfg.n_sources = 1;
+        cfg.sources = & src;
+        cfg.max_scatter = 100;
+        cfg.max_steps = 100000;
+        cfg.fx_shift = 32;
+        cfg.n_batches = cfg.image_batch_n = 1;
+        cfg.image_n = image ? 32 : 0;
+        cfg.image_half_width = 1;
+        cfg.inclination_deg = 60;
+        cfg.image_center[ 0 ] = cfg.image_center[ 1 ] = cfg.image_center[ 2 ] = 0.5;
+        t.image = t.image_batch = ( void * ) 4096;
+    }
+    int run( kp_mesh_t * m, cudaStream_t s = nullptr ) { return kp_transport_forward( m, & cfg, & t, s ); }
+    long long tape( kp_mesh_t * m )
+    {
+        long long id = 0;
+        expect( kp_transport_forward_tape( m, & cfg, & t, nullptr, & id ) == KP_OK && id > 0, "taped solve" );
+        return id;
+    }
+    int adjoint_tape( kp_mesh_t * m, long long id )
+    { return kp_transport_adjoint_tape( m, id, & cfg, ( float * ) 4096, 24, ( void * ) 4096, ( void * ) 4096, nullptr, nullptr ); }
+};
+
+// A uniform mesh of n^3 cells in blocks of 16^3.
+kp_mesh_t * make_mesh( int n )
+{
+    kp_mesh_desc_t d {  };
+    for( int a = 0; a < 3; ++ a )
+    {
+        d.x_max[ a ] = 1;
+        d.n_cell_global[ a ] = n;
+        d.n_cell_block[ a ] = 16;
+    }
+    kp_mesh_t * m = nullptr;
+    expect( kp_mesh_create( & d, & m ) == KP_OK, "mesh" );
+    return m;
+}
+
+// The gradient of a taped solve has room for its walk's packets, or an error.
+void tape_pool(  )
+{
+    kp_mesh_t * m = make_mesh( 32 );
+    solve_t taped( 2000, true ), plain( 100000, false );
+    const long long id = taped.tape( m );
+    F.limit = 0;                         // the device is full, another program's what is freed
+    expect( plain.run( m ) != KP_OK, "a solve without memory" );
+    F.launches.clear(  );
+    const int r = taped.adjoint_tape( m, id );
+    bool walked = false;
+    for( const auto & l : F.launches )
+        if( l.kernel.find( "k_walk" ) != std::string::npos )
+            walked = l.P.pool != nullptr && l.P.pool_n > 0;
+    expect( r != KP_OK || walked, "adjoint without a pool" );
+    kp_mesh_destroy( m );
+}
+}   // namespace
+
+int main( int argc, char ** argv )
+{
+    const std::string what = argc > 1 ? argv[ 1 ] : "";
+    if( what == "tape_pool" ) tape_pool(  );
+    else return 2;
+    if( fails == 0 ) std::printf( "OK %s\n", what.c_str(  ) );
+    return fails != 0;
+}
