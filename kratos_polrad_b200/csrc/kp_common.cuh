@@ -105,9 +105,9 @@ struct pool_mem_t
     pool_mem_t & operator=( const pool_mem_t & ) = delete;
     ~ pool_mem_t(  ) { release(  ); }
     void release(  )
-    {
-        cudaFree( d );
-        cudaFree( old );
+    {   // (a free of null would make a context, also for a mesh of the host)
+        if( d ) cudaFree( d );
+        if( old ) cudaFree( old );
         d = old = nullptr;
         bytes = 0;
         captured = full = false;

@@ -187,6 +187,14 @@ kp_mesh_t * make_mesh( int n )
     return m;
 }
 
+// A mesh that was never on a device comes and goes without the runtime, whose
+// first call (a free of null is one) would make a context.
+void host_mesh(  )
+{
+    kp_mesh_destroy( make_mesh( 32 ) );
+    expect( F.calls == 0, "a host mesh calls the runtime" );
+}
+
 // The gradient of a taped solve has room for its walk's packets, or an error.
 void tape_pool(  )
 {
@@ -209,7 +217,8 @@ void tape_pool(  )
 int main( int argc, char ** argv )
 {
     const std::string what = argc > 1 ? argv[ 1 ] : "";
-    if( what == "tape_pool" ) tape_pool(  );
+    if( what == "host_mesh" ) host_mesh(  );
+    else if( what == "tape_pool" ) tape_pool(  );
     else return 2;
     if( fails == 0 ) std::printf( "OK %s\n", what.c_str(  ) );
     return fails != 0;
