@@ -383,7 +383,9 @@ typedef struct kp_tallies
  * queue).  With an image, the first solve of a mesh allocates its peel-off
  * queue: 64 B per ray, 12 rays per packet, at most kp_mesh_peel_queue_limit
  * rays (default 2^27, 8.6 GB); later solves reuse it, and the mesh frees it
- * with the mesh. */
+ * with the mesh.  A solve that is captured into a graph needs a queue that is
+ * large enough already; what it was given stays allocated until the mesh goes,
+ * also where a later solve outgrows it. */
 int kp_transport_forward( kp_mesh_t * mesh, const kp_transport_cfg_t * cfg,
                           const kp_tallies_t * tallies, void * stream );
 

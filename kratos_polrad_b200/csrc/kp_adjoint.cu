@@ -498,7 +498,7 @@ void adjoint_buffers( kp_mesh_t * mesh, fwd_params_t & P, long long n_pk )
                                + 255 ) & ~( size_t ) 255;
     if( mesh->adj_bytes < adj_bytes + priv_bytes )
     {
-        cudaFree( mesh->d_adj );
+        mesh->drop( mesh->d_adj, mesh->adj_captured );
         mesh->d_adj = nullptr;
         mesh->adj_bytes = 0;
         mesh->tape_id = 0;
@@ -631,6 +631,7 @@ extern "C" int kp_transport_adjoint( kp_mesh_t * mesh, const kp_transport_cfg_t 
         kp::ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
         // both marches read the queue in the forward solve's order
         int * perm = kp::march_order( mesh, P.n_packets, s );
+        mesh->note_capture( s );
         static thread_local kp::fwd_params_t C;
         for( long long done = 0; done < P.n_packets; done += chunk )
         {
@@ -683,6 +684,7 @@ extern "C" int kp_transport_forward_tape( kp_mesh_t * mesh, const kp_transport_c
         P.pq_perm = kp::march_order( mesh, P.n_packets, ( cudaStream_t ) stream );
         const bool sorted = P.pq_perm != nullptr;
         auto s = ( cudaStream_t ) stream;
+        mesh->note_capture( s );
         KP_CUDA( cudaMemsetAsync( P.work, 0, 4 * sizeof( unsigned long long ), s ) );
         KP_CUDA( cudaMemsetAsync( P.adj_head, 0xff, P.n_packets * sizeof( int ), s ) );
         KP_CUDA( cudaMemsetAsync( P.adj_flag, 0, P.n_packets * sizeof( int ), s ) );
@@ -724,6 +726,7 @@ extern "C" int kp_transport_adjoint_tape( kp_mesh_t * mesh, long long tape_id,
         // a solve without an image since then leaves the tape, but may have
         // lost the pool for want of memory
         kp::ensure_pool( mesh->pool, mesh->tape_n, s );
+        mesh->note_capture( s );
         mesh->refresh_ext( s );
         const unsigned gs = 4 * 148;
         kp::k_adj_score<<< gs, 256, 0, s >>>( P );                        // G from the tape

@@ -12,6 +12,7 @@
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <vector>
 
 namespace kp
 {
@@ -92,6 +93,14 @@ struct alignas( 16 ) blk_meta_t
 };
 static_assert( sizeof( blk_meta_t ) == 16, "meta record" );
 
+// Whether stream s is being captured.
+inline bool capturing( cudaStream_t s )
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    KP_CUDA( cudaStreamIsCapturing( s, & st ) );
+    return st != cudaStreamCaptureStatusNone;
+}
+
 // Device memory of the walk's packet pools (kp_walk.cu).
 struct pool_mem_t
 {
@@ -170,6 +179,11 @@ struct kp_mesh
     void       * d_sort_tmp = nullptr;
     size_t       sort_cells = 0, sort_perm = 0, sort_tmp_bytes = 0;
     void       * d_adj   = nullptr;  size_t adj_bytes = 0;      // deferred adjoint
+    // Which of d_pq, d_sort_perm and d_adj a captured solve was given.  Such a
+    // buffer, when a later solve outgrows it, is kept in `kept` until the mesh
+    // goes: the capture's replays still use it.
+    bool         pq_captured = false, perm_captured = false, adj_captured = false;
+    std::vector< void * > kept;
     // the taped forward solve whose rays the queue and d_adj hold (0: none)
     long long    tape_id = 0, tape_serial = 0;
     long long    tape_n  = 0;                                      // its packets
@@ -191,6 +205,10 @@ struct kp_mesh
     // Recomputes d_ext from d_sigma on stream s: every solve does this first,
     // since callers may write the coefficients through kp_mesh_sigma_ptr.
     void refresh_ext( cudaStream_t s );
+    // Gives back a buffer, or keeps it when a captured solve was given it; the
+    // other marks the buffers that a solve on s was given, if s is captured.
+    void drop( void * p, bool & was_captured );
+    void note_capture( cudaStream_t s );
     void release(  );
 };
 

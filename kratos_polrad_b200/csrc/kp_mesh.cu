@@ -177,8 +177,23 @@ void kp_mesh::upload( bool with_sigma )
     uploaded = true;
 }
 
+void kp_mesh::drop( void * p, bool & was_captured )
+{
+    if( p && was_captured ) kept.push_back( p );
+    else                    KP_CUDA( cudaFree( p ) );
+    was_captured = false;
+}
+
+void kp_mesh::note_capture( cudaStream_t s )
+{
+    if( kp::capturing( s ) ) pq_captured = perm_captured = adj_captured = true;
+}
+
 void kp_mesh::release(  )
 {
+    for( void * p : kept ) cudaFree( p );
+    kept.clear(  );
+    pq_captured = perm_captured = adj_captured = false;
     cudaFree( d_nb );     d_nb     = nullptr;
     cudaFree( d_meta );   d_meta   = nullptr;
     cudaFree( d_geo_d );  d_geo_d  = nullptr;

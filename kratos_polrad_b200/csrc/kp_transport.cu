@@ -1285,9 +1285,7 @@ void begin_flux( kp_mesh_t * mesh, const kp_tallies_t & t, int tally_mode, fwd_p
     const size_t bytes = ( size_t ) P.m.n_blocks * P.m.cpb * sizeof( double );
     if( mesh->d_flux == nullptr )
     {
-        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        KP_CUDA( cudaStreamIsCapturing( s, & st ) );
-        if( st != cudaStreamCaptureStatusNone ) return;
+        if( capturing( s ) ) return;
         if( cudaMalloc( & mesh->d_flux, bytes ) != cudaSuccess )
         {
             cudaGetLastError(  );
@@ -1403,7 +1401,7 @@ void ensure_peel_queue( kp_mesh_t * mesh, long long n_packets )
                                      mesh->pq_limit );
     if( mesh->pq_cap < want )
     {
-        cudaFree( mesh->d_pq );
+        mesh->drop( mesh->d_pq, mesh->pq_captured );
         mesh->d_pq = nullptr;
         mesh->pq_cap = 0;
         KP_CUDA( cudaMalloc( & mesh->d_pq, ( size_t ) want * sizeof( peel_task_t ) ) );
@@ -1455,7 +1453,7 @@ int * ensure_task_sort( kp_mesh_t * mesh, long long pq_cap )
     }
     if( mesh->sort_perm < n_slots )
     {
-        cudaFree( mesh->d_sort_perm );
+        mesh->drop( mesh->d_sort_perm, mesh->perm_captured );
         mesh->d_sort_perm = nullptr;
         mesh->sort_perm = 0;
         KP_CUDA( cudaMalloc( & mesh->d_sort_perm, n_slots * sizeof( int ) ) );
@@ -1474,9 +1472,7 @@ int * march_order( kp_mesh_t * mesh, long long n, cudaStream_t s )
     if( ! peel_sorted( mesh, 0 ) )
     {
         const auto v = mesh->view(  );
-        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        KP_CUDA( cudaStreamIsCapturing( s, & st ) );
-        if( st != cudaStreamCaptureStatusNone
+        if( capturing( s )
             && ( mesh->sort_cells < ( size_t ) v.n_blocks * v.cpb
                  || mesh->sort_perm < ( size_t ) mesh->pq_cap + 32 ) )
             return nullptr;
@@ -1559,6 +1555,7 @@ void launch_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s )
     const long long chunk = std::max< long long >( mesh->pq_cap / PQ_PER_PACKET, 1 );
     ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
     int * perm = march_order( mesh, P.n_packets, s );
+    mesh->note_capture( s );
     static thread_local fwd_params_t C;
     for( long long done = 0; done < P.n_packets; done += chunk )
     {
@@ -1621,10 +1618,10 @@ extern "C" int kp_mesh_peel_queue_limit( kp_mesh_t * mesh, long long max_rays )
                      KP_ERR_CONFIG );
         if( mesh->pq_cap > max_rays )
         {   // the next solve allocates a queue within the new limit
-            KP_CUDA( cudaFree( mesh->d_pq ) );
+            mesh->drop( mesh->d_pq, mesh->pq_captured );
             mesh->d_pq = nullptr;
             mesh->pq_cap = 0;
-            KP_CUDA( cudaFree( mesh->d_adj ) );
+            mesh->drop( mesh->d_adj, mesh->adj_captured );
             mesh->d_adj = nullptr;
             mesh->adj_bytes = 0;
             mesh->tape_id = 0;
@@ -1673,6 +1670,7 @@ void launch_resume_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStrea
     const long long chunk = std::max< long long >( mesh->pq_cap / PQ_PER_PACKET, 1 );
     ensure_pool( mesh->pool, std::min( chunk, items ), s );
     int * perm = march_order( mesh, items, s );
+    mesh->note_capture( s );
     static thread_local fwd_params_t C;
     for( long long lo = 0; lo < items; lo += chunk )
     {

@@ -866,9 +866,7 @@ void ensure_pool( pool_mem_t & mem, long long items, cudaStream_t s )
     int dev = 0, n_sm = 0;
     KP_CUDA( cudaGetDevice( & dev ) );
     KP_CUDA( cudaDeviceGetAttribute( & n_sm, cudaDevAttrMultiProcessorCount, dev ) );
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    KP_CUDA( cudaStreamIsCapturing( s, & st ) );
-    const bool capturing = st != cudaStreamCaptureStatusNone;
+    const bool in_capture = capturing( s );
     const long long warps = ( long long ) n_sm * KP_WALK_MINB * WALK_WARPS;
     auto bytes = [ & ]( long long n )
     {
@@ -881,7 +879,7 @@ void ensure_pool( pool_mem_t & mem, long long items, cudaStream_t s )
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;     // for this thread's allocation
         KP_CUDA( cudaThreadExchangeStreamCaptureMode( & mode ) );
         void * d = nullptr;
-        const bool keep = mem.captured || ( capturing && mem.d );
+        const bool keep = mem.captured || ( in_capture && mem.d );
         if( ! keep )
         {
             cudaFree( mem.d );
@@ -914,7 +912,7 @@ void ensure_pool( pool_mem_t & mem, long long items, cudaStream_t s )
             KP_CUDA( e );
         }
     }
-    mem.captured = mem.captured || capturing;
+    mem.captured = mem.captured || in_capture;
 }
 
 void launch_walk( fwd_params_t & P, pool_mem_t & mem, int tally_mode, walk_kind kind, cudaStream_t s,

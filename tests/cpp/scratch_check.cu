@@ -51,6 +51,15 @@ cudaError_t ret( cudaError_t e )
     return e;
 }
 
+// The allocation that holds address a (0: none).
+uintptr_t owner( uintptr_t a )
+{
+    auto it = F.live.upper_bound( a );
+    if( it == F.live.begin(  ) ) return 0;
+    -- it;
+    return a < it->first + it->second ? it->first : 0;
+}
+
 int fails = 0;
 void expect( bool ok, const char * what )
 {
@@ -168,6 +177,8 @@ struct solve_t
         expect( kp_transport_forward_tape( m, & cfg, & t, nullptr, & id ) == KP_OK && id > 0, "taped solve" );
         return id;
     }
+    int adjoint( kp_mesh_t * m, cudaStream_t s )
+    { return kp_transport_adjoint( m, & cfg, ( float * ) 4096, 24, ( void * ) 4096, ( void * ) 4096, nullptr, s ); }
     int adjoint_tape( kp_mesh_t * m, long long id )
     { return kp_transport_adjoint_tape( m, id, & cfg, ( float * ) 4096, 24, ( void * ) 4096, ( void * ) 4096, nullptr, nullptr ); }
 };
@@ -212,6 +223,55 @@ void tape_pool(  )
     expect( r != KP_OK || walked, "adjoint without a pool" );
     kp_mesh_destroy( m );
 }
+// The allocations that the launches so far were given.
+std::set< uintptr_t > given(  )
+{
+    std::set< uintptr_t > r;
+    for( const auto & l : F.launches )
+    {
+        std::vector< uintptr_t > w( sizeof( l.P ) / sizeof( uintptr_t ) );
+        std::memcpy( w.data(  ), & l.P, w.size(  ) * sizeof( uintptr_t ) );
+        for( void * a : l.args ) w.push_back( ( uintptr_t ) a );
+        for( uintptr_t a : w ) if( owner( a ) ) r.insert( owner( a ) );
+    }
+    return r;
+}
+
+// What a captured solve was given stays allocated, through larger solves and a
+// lower queue limit, until its mesh goes; the larger solves' own buffers are
+// not kept beside it.
+void captured(  )
+{
+    const cudaStream_t S = ( cudaStream_t ) 64;
+    for( int kind = 0; kind < 4; ++ kind )           // as queued, by cell, adjoint, no image
+    {
+        kp_mesh_t * m = make_mesh( 32 );
+        if( kind == 1 ) kp_mesh_peel_order( m, KP_PEEL_ORDER_CELL );
+        auto solve = [ & ]( long long n )
+        {
+            solve_t s( n, kind != 3 );
+            return kind == 2 ? s.adjoint( m, S ) : s.run( m, S );
+        };
+        expect( solve( 20000 ) == KP_OK, "solve" );
+        F.capturing = S;
+        F.launches.clear(  );
+        expect( solve( 20000 ) == KP_OK && ! F.broken, "captured solve" );
+        F.capturing = nullptr;
+        const auto held = given(  );
+        size_t n_live = 0;
+        for( int k = 0; k < 3; ++ k )
+        {
+            expect( solve( 100000 << k ) == KP_OK, "larger solve" );
+            if( k > 0 ) expect( F.live.size(  ) <= n_live, "outgrown buffers pile up" );
+            n_live = F.live.size(  );
+        }
+        expect( kp_mesh_peel_queue_limit( m, 5000 ) == KP_OK && solve( 1000 ) == KP_OK, "lower limit" );
+        for( uintptr_t a : held )
+            expect( F.live.count( a ) != 0, "a captured solve's memory was freed" );
+        kp_mesh_destroy( m );
+        expect( F.live.empty(  ), "memory left behind" );
+    }
+}
 }   // namespace
 
 int main( int argc, char ** argv )
@@ -219,6 +279,7 @@ int main( int argc, char ** argv )
     const std::string what = argc > 1 ? argv[ 1 ] : "";
     if( what == "host_mesh" ) host_mesh(  );
     else if( what == "tape_pool" ) tape_pool(  );
+    else if( what == "captured" ) captured(  );
     else return 2;
     if( fails == 0 ) std::printf( "OK %s\n", what.c_str(  ) );
     return fails != 0;
