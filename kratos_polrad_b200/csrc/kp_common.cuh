@@ -101,6 +101,18 @@ inline bool capturing( cudaStream_t s )
     return st != cudaStreamCaptureStatusNone;
 }
 
+// For an allocation (or a free) that a solve makes for speed alone: while a
+// relaxed_t lives, this thread's calls disturb no capture, its own or, in the
+// global mode, another thread's.
+struct relaxed_t
+{
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    relaxed_t(  )  { KP_CUDA( cudaThreadExchangeStreamCaptureMode( & mode ) ); }
+    ~ relaxed_t(  ) { cudaThreadExchangeStreamCaptureMode( & mode ); }
+    relaxed_t( const relaxed_t & ) = delete;
+    relaxed_t & operator=( const relaxed_t & ) = delete;
+};
+
 // Device memory of the walk's packet pools (kp_walk.cu).
 struct pool_mem_t
 {

@@ -1264,9 +1264,9 @@ void fold_carry( const kp_transport_cfg_t & c, const kp_tallies_t & t, cudaStrea
 // and a second one for what it rounded off.  A solve of a mesh sums in double
 // instead, one reduction per segment, and rounds once at its end: 1e6 packets,
 // 128^3 root, inclination 60: walk 7.6 -> 5.9 ms, solve 14.8 -> 13.2 ms.
-// The array (8 bytes per cell) belongs to the mesh; where it cannot be had (a
-// capture before the mesh's first such solve, no memory left), the deposits
-// go to the tally and its carry.
+// The array (8 bytes per cell) belongs to the mesh and is allocated by its
+// first such solve, captured or not; where there is no memory for it, the
+// deposits go to the tally and its carry.
 __global__ void k_fold_flux( const double * __restrict__ sum, float * __restrict__ flux, long long n )
 {
     for( long long i = ( long long ) blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -1285,7 +1285,7 @@ void begin_flux( kp_mesh_t * mesh, const kp_tallies_t & t, int tally_mode, fwd_p
     const size_t bytes = ( size_t ) P.m.n_blocks * P.m.cpb * sizeof( double );
     if( mesh->d_flux == nullptr )
     {
-        if( capturing( s ) ) return;
+        const relaxed_t relaxed;
         if( cudaMalloc( & mesh->d_flux, bytes ) != cudaSuccess )
         {
             cudaGetLastError(  );
@@ -1476,6 +1476,7 @@ int * march_order( kp_mesh_t * mesh, long long n, cudaStream_t s )
             && ( mesh->sort_cells < ( size_t ) v.n_blocks * v.cpb
                  || mesh->sort_perm < ( size_t ) mesh->pq_cap + 32 ) )
             return nullptr;
+        const relaxed_t relaxed;
         try
         {
             return ensure_task_sort( mesh, mesh->pq_cap );

@@ -876,8 +876,7 @@ void ensure_pool( pool_mem_t & mem, long long items, cudaStream_t s )
     size_t want = bytes( items );
     if( mem.bytes < want && ! mem.full )
     {
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;     // for this thread's allocation
-        KP_CUDA( cudaThreadExchangeStreamCaptureMode( & mode ) );
+        const relaxed_t relaxed;
         void * d = nullptr;
         const bool keep = mem.captured || ( in_capture && mem.d );
         if( ! keep )
@@ -896,7 +895,6 @@ void ensure_pool( pool_mem_t & mem, long long items, cudaStream_t s )
             want /= 2;
             e = cudaMalloc( & d, want );
         }
-        cudaThreadExchangeStreamCaptureMode( & mode );
         if( e == cudaSuccess )
         {
             if( keep ) mem.old = mem.d;

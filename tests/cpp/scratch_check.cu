@@ -170,6 +170,14 @@ struct solve_t
         cfg.image_center[ 0 ] = cfg.image_center[ 1 ] = cfg.image_center[ 2 ] = 0.5;
         t.image = t.image_batch = ( void * ) 4096;
     }
+    // a float flux with its carry, on a mesh of n cells
+    solve_t & flux( long long n )
+    {
+        cfg.tally_mode = KP_TALLY_FLOAT;
+        t.flux = t.carry = ( float * ) 4096;
+        t.flux_n = n;
+        return * this;
+    }
     int run( kp_mesh_t * m, cudaStream_t s = nullptr ) { return kp_transport_forward( m, & cfg, & t, s ); }
     long long tape( kp_mesh_t * m )
     {
@@ -272,6 +280,41 @@ void captured(  )
         expect( F.live.empty(  ), "memory left behind" );
     }
 }
+// What a solve allocates beside its queue, for speed alone, disturbs no capture
+// under way in another thread, and a captured solve has it too.
+void other_capture(  )
+{
+    kp_mesh_t * m = make_mesh( 160 );                // 16 MB of extinction: sorted by the packet count
+    solve_t s( 500000, true );
+    kp_mesh_peel_order( m, KP_PEEL_ORDER_QUEUE );
+    expect( s.run( m ) == KP_OK, "solve as queued" );
+    kp_mesh_peel_order( m, KP_PEEL_ORDER_AUTO );
+    F.other_captures = true;
+    F.launches.clear(  );
+    expect( s.run( m ) == KP_OK && ! F.broken, "the march order's buffers" );
+    bool sorted = false;
+    for( const auto & l : F.launches ) sorted = sorted || l.kernel.find( "k_task_sort" ) != std::string::npos;
+    expect( sorted, "marched by cell" );
+    F.other_captures = false;
+    kp_mesh_destroy( m );
+
+    for( const cudaStream_t S : { ( cudaStream_t ) nullptr, ( cudaStream_t ) 64 } )
+    {
+        m = make_mesh( 32 );
+        solve_t f( 2000, false );
+        expect( f.run( m ) == KP_OK, "solve" );
+        F.capturing = S;                             // itself captured, or beside a capture
+        F.other_captures = S == nullptr;
+        F.launches.clear(  );
+        f.flux( 32768 );
+        expect( f.run( m, S ) == KP_OK && ! F.broken, "the flux sums" );
+        for( const auto & l : F.launches )
+            expect( l.kernel.find( "k_walk" ) == std::string::npos || l.P.flux_sum, "flux in double" );
+        F.capturing = nullptr;
+        F.other_captures = false;
+        kp_mesh_destroy( m );
+    }
+}
 }   // namespace
 
 int main( int argc, char ** argv )
@@ -280,6 +323,7 @@ int main( int argc, char ** argv )
     if( what == "host_mesh" ) host_mesh(  );
     else if( what == "tape_pool" ) tape_pool(  );
     else if( what == "captured" ) captured(  );
+    else if( what == "other_capture" ) other_capture(  );
     else return 2;
     if( fails == 0 ) std::printf( "OK %s\n", what.c_str(  ) );
     return fails != 0;

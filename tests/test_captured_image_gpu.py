@@ -1,4 +1,4 @@
-"""Captured solves with an image, and captured gradients, replayed after larger
+"""Captured solves with an image and captured gradients, replayed after larger
 solves of the same mesh: the queue, the march order and the adjoint's buffers
 that the capture was given are still theirs.  int64 tallies: no tolerance."""
 import dataclasses
@@ -9,7 +9,7 @@ import torch
 
 from kratos_polrad_b200.adjoint import adjoint
 from kratos_polrad_b200.mesh import PEEL_ORDER_AUTO, PEEL_ORDER_CELL
-from kratos_polrad_b200.transport import Tallies, forward
+from kratos_polrad_b200.transport import TALLY_FLOAT, Tallies, forward
 from transport_cases import case
 
 pytestmark = pytest.mark.gpu
@@ -52,3 +52,28 @@ def test_captured_gradient_survives_a_larger_one():
     assert mesh.status() == 0
     for x, y in zip(got, want):
         assert y.abs().sum() > 0 and torch.equal(x, y)
+
+
+def test_captured_float_flux_before_any_other():
+    """The mesh's first float flux, captured and replayed twice: summed in
+    double and rounded once per replay, so within 2 * 2^-24 of the fixed-point
+    sums, plus those sums' half a unit per segment."""
+    mesh, sig, t = case("slab")
+    mesh.set_sigma(sig)
+    t = dataclasses.replace(t, n_packets=20_000, n_record=0, flux=True, flux_fx_shift=30)
+    fx = Tallies(t, n_cells=mesh.n_cells)
+    forward(mesh, t, fx)
+    forward(mesh, t, fx)
+    tf = dataclasses.replace(t, tally_mode=TALLY_FLOAT)
+    fl = Tallies(tf, n_cells=mesh.n_cells)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        forward(mesh, tf, fl)
+    g.replay()
+    g.replay()
+    torch.cuda.synchronize()
+    assert mesh.status() == 0
+    want = fx.flux.double() * fx.flux_scale()
+    steps = fx.counts()["steps"]
+    assert want.max() > 0
+    assert ((fl.flux.double() - want).abs() <= 2 * 2.0 ** -24 * want + steps * 2.0 ** -31).all()
