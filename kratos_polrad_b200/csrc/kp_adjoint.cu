@@ -502,7 +502,7 @@ void adjoint_buffers( kp_mesh_t * mesh, fwd_params_t & P, long long n_pk )
         mesh->d_adj = nullptr;
         mesh->adj_bytes = 0;
         mesh->tape_id = 0;
-        KP_CUDA( cudaMalloc( & mesh->d_adj, adj_bytes + priv_bytes ) );
+        mesh->need( & mesh->d_adj, adj_bytes + priv_bytes );
         mesh->adj_bytes = adj_bytes + priv_bytes;
     }
     char * a = static_cast< char * >( mesh->d_adj );
@@ -628,9 +628,9 @@ extern "C" int kp_transport_adjoint( kp_mesh_t * mesh, const kp_transport_cfg_t 
         kp::ensure_peel_queue( mesh, P.n_packets );
         const long long chunk = std::max< long long >( mesh->pq_cap / kp::PQ_PER_PACKET, 1 );
         kp::adjoint_buffers( mesh, P, std::min( chunk, P.n_packets ) );
-        kp::ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
         // both marches read the queue in the forward solve's order
         int * perm = kp::march_order( mesh, P.n_packets, s );
+        kp::ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
         mesh->note_capture( s );
         static thread_local kp::fwd_params_t C;
         for( long long done = 0; done < P.n_packets; done += chunk )
@@ -670,25 +670,24 @@ extern "C" int kp_transport_forward_tape( kp_mesh_t * mesh, const kp_transport_c
         if( P.n_packets > std::max< long long >( mesh->pq_cap / kp::PQ_PER_PACKET, 1 ) )
         {   // more packets than one chunk of the queue: an untaped solve
             P.work = mesh->workspace(  );
-            kp::begin_flux( mesh, * tallies, cfg->tally_mode, P, ( cudaStream_t ) stream );
             kp::launch_deferred_solve( mesh, P, cfg->tally_mode, ( cudaStream_t ) stream );
             kp::fold_flux( P, ( cudaStream_t ) stream );
             kp::fold_carry( * cfg, * tallies, ( cudaStream_t ) stream );
             return;
         }
         kp::adjoint_buffers( mesh, P, P.n_packets );
-        kp::ensure_pool( mesh->pool, P.n_packets, ( cudaStream_t ) stream );
         // the march order; the gradient's depositing march reads the same
         // permutation, which lives as long as the tape (every solve that
         // overwrites the queue drops the tape)
         P.pq_perm = kp::march_order( mesh, P.n_packets, ( cudaStream_t ) stream );
         const bool sorted = P.pq_perm != nullptr;
         auto s = ( cudaStream_t ) stream;
+        kp::ensure_pool( mesh->pool, P.n_packets, s );
+        kp::begin_flux( mesh, cfg->tally_mode, P, s );
         mesh->note_capture( s );
         KP_CUDA( cudaMemsetAsync( P.work, 0, 4 * sizeof( unsigned long long ), s ) );
         KP_CUDA( cudaMemsetAsync( P.adj_head, 0xff, P.n_packets * sizeof( int ), s ) );
         KP_CUDA( cudaMemsetAsync( P.adj_flag, 0, P.n_packets * sizeof( int ), s ) );
-        kp::begin_flux( mesh, * tallies, cfg->tally_mode, P, s );
         if( cfg->tally_mode == KP_TALLY_FIXED )
             kp::launch_deferred_chunk< KP_TALLY_FIXED, true >( P, s, mesh );
         else

@@ -119,7 +119,7 @@ struct pool_mem_t
     void * d = nullptr;
     size_t bytes = 0;
     void * old = nullptr;                 // an outgrown pool that a captured launch uses
-    bool   captured = false, full = false;
+    bool   captured = false, full = false;     // d is in a captured launch; of the full size
 
     pool_mem_t(  ) = default;
     pool_mem_t( const pool_mem_t & ) = delete;
@@ -195,6 +195,7 @@ struct kp_mesh
     // buffer, when a later solve outgrows it, is kept in `kept` until the mesh
     // goes: the capture's replays still use it.
     bool         pq_captured = false, perm_captured = false, adj_captured = false;
+    bool         sort_captured = false;      // ... and of the sort's other buffers, d_flux
     std::vector< void * > kept;
     // the taped forward solve whose rays the queue and d_adj hold (0: none)
     long long    tape_id = 0, tape_serial = 0;
@@ -220,12 +221,21 @@ struct kp_mesh
     // Gives back a buffer, or keeps it when a captured solve was given it; the
     // other marks the buffers that a solve on s was given, if s is captured.
     void drop( void * p, bool & was_captured );
+    // Memory that a solve cannot do without.  Where there is too little, the
+    // mesh first gives back what it keeps for speed alone: the packet pool, the
+    // flux sums and an order that only the packet count asked for.  A solve
+    // makes those last, as large as still fits.
+    void need( void ** p, size_t bytes );
     void note_capture( cudaStream_t s );
+    void release_sort(  );
     void release(  );
 };
 
 namespace kp
 {
+// Whether a solve of n packets marches the mesh's queue sorted by starting
+// cell (kp_mesh_peel_order); n = 0: whatever its packet count.
+bool peel_sorted( const kp_mesh * mesh, long long n );
 // ext[i] = sigma[i].x + sigma[i].y (IEEE float add) for n cells, on stream s.
 void extinction( const float2 * sigma, float * ext, long long n, cudaStream_t s );
 }

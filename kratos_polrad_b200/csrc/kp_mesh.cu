@@ -184,16 +184,43 @@ void kp_mesh::drop( void * p, bool & was_captured )
     was_captured = false;
 }
 
+void kp_mesh::need( void ** p, size_t bytes )
+{
+    cudaError_t e = cudaMalloc( p, bytes );
+    if( e == cudaErrorMemoryAllocation )
+    {
+        cudaGetLastError(  );
+        if( ! pool.captured ) pool.release(  );
+        if( ! sort_captured )
+        {
+            cudaFree( d_flux );
+            d_flux = nullptr;
+            if( ! kp::peel_sorted( this, 0 ) && ! ( tape_id && tape_sorted ) ) release_sort(  );
+        }
+        e = cudaMalloc( p, bytes );
+    }
+    KP_CUDA( e );
+}
+
 void kp_mesh::note_capture( cudaStream_t s )
 {
-    if( kp::capturing( s ) ) pq_captured = perm_captured = adj_captured = true;
+    if( kp::capturing( s ) ) pq_captured = perm_captured = adj_captured = sort_captured = true;
+}
+
+void kp_mesh::release_sort(  )
+{
+    cudaFree( d_sort_cnt );  d_sort_cnt  = nullptr;
+    cudaFree( d_sort_off );  d_sort_off  = nullptr;
+    cudaFree( d_sort_perm ); d_sort_perm = nullptr;
+    cudaFree( d_sort_tmp );  d_sort_tmp  = nullptr;
+    sort_cells = sort_perm = sort_tmp_bytes = 0;
 }
 
 void kp_mesh::release(  )
 {
     for( void * p : kept ) cudaFree( p );
     kept.clear(  );
-    pq_captured = perm_captured = adj_captured = false;
+    pq_captured = perm_captured = adj_captured = sort_captured = false;
     cudaFree( d_nb );     d_nb     = nullptr;
     cudaFree( d_meta );   d_meta   = nullptr;
     cudaFree( d_geo_d );  d_geo_d  = nullptr;
@@ -206,11 +233,7 @@ void kp_mesh::release(  )
     pool.release(  );
     cudaFree( d_flux );   d_flux   = nullptr;
     cudaFree( d_pq );     d_pq     = nullptr; pq_cap = 0;
-    cudaFree( d_sort_cnt );  d_sort_cnt  = nullptr;
-    cudaFree( d_sort_off );  d_sort_off  = nullptr;
-    cudaFree( d_sort_perm ); d_sort_perm = nullptr;
-    cudaFree( d_sort_tmp );  d_sort_tmp  = nullptr;
-    sort_cells = sort_perm = sort_tmp_bytes = 0;
+    release_sort(  );
     cudaFree( d_adj );    d_adj    = nullptr; adj_bytes = 0; tape_id = 0;
     cudaFree( d_rf_f );   d_rf_f   = nullptr;
     cudaFree( d_rf_d );   d_rf_d   = nullptr;

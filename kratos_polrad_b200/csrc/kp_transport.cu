@@ -1277,10 +1277,9 @@ __global__ void k_fold_flux( const double * __restrict__ sum, float * __restrict
     }
 }
 
-void begin_flux( kp_mesh_t * mesh, const kp_tallies_t & t, int tally_mode, fwd_params_t & P,
-                 cudaStream_t s )
+void begin_flux( kp_mesh_t * mesh, int tally_mode, fwd_params_t & P, cudaStream_t s )
 {
-    if( tally_mode != KP_TALLY_FLOAT || t.flux == nullptr || P.c_flux == nullptr )
+    if( tally_mode != KP_TALLY_FLOAT || P.flux == nullptr || P.c_flux == nullptr )
         return;
     const size_t bytes = ( size_t ) P.m.n_blocks * P.m.cpb * sizeof( double );
     if( mesh->d_flux == nullptr )
@@ -1404,7 +1403,7 @@ void ensure_peel_queue( kp_mesh_t * mesh, long long n_packets )
         mesh->drop( mesh->d_pq, mesh->pq_captured );
         mesh->d_pq = nullptr;
         mesh->pq_cap = 0;
-        KP_CUDA( cudaMalloc( & mesh->d_pq, ( size_t ) want * sizeof( peel_task_t ) ) );
+        mesh->need( & mesh->d_pq, ( size_t ) want * sizeof( peel_task_t ) );
         mesh->pq_cap = want;
     }
 }
@@ -1417,7 +1416,7 @@ void ensure_peel_queue( kp_mesh_t * mesh, long long n_packets )
 // gradient of 1e6 packets, 24.9 and 22.5; 20 MB 13.5 and 12.9; 32 MB 15.4 and
 // 14.6, and 1e5 packets 2.57 and 2.52, which the sort's buffers, about 1 ms on a
 // mesh's first such solve, outweigh; 51 MB 18.1 and 16.8; 74 MB 20.3 and 18.8.
-bool peel_sorted( const kp_mesh_t * mesh, long long n )
+bool peel_sorted( const kp_mesh * mesh, long long n )
 {
     if( mesh->peel_order != KP_PEEL_ORDER_AUTO )
         return mesh->peel_order == KP_PEEL_ORDER_CELL;
@@ -1428,9 +1427,15 @@ bool peel_sorted( const kp_mesh_t * mesh, long long n )
 }
 
 // Makes room on the mesh for sorting a queue of pq_cap tasks (a permutation
-// of pq_cap + 32 slots: whole groups of 32); returns the permutation.
-int * ensure_task_sort( kp_mesh_t * mesh, long long pq_cap )
+// of pq_cap + 32 slots: whole groups of 32); returns the permutation.  must:
+// the solve has no other order.
+int * ensure_task_sort( kp_mesh_t * mesh, long long pq_cap, bool must )
 {
+    auto get = [ & ]( void ** p, size_t bytes )
+    {
+        if( must ) mesh->need( p, bytes );
+        else       KP_CUDA( cudaMalloc( p, bytes ) );
+    };
     const auto v = mesh->view(  );
     const size_t nk = ( size_t ) v.n_blocks * v.cpb;
     const size_t n_slots = ( size_t ) pq_cap + 32;
@@ -1442,12 +1447,12 @@ int * ensure_task_sort( kp_mesh_t * mesh, long long pq_cap )
         mesh->d_sort_cnt = mesh->d_sort_off = nullptr;
         mesh->d_sort_tmp = nullptr;
         mesh->sort_cells = mesh->sort_tmp_bytes = 0;
-        KP_CUDA( cudaMalloc( & mesh->d_sort_cnt, nk * sizeof( unsigned ) ) );
-        KP_CUDA( cudaMalloc( & mesh->d_sort_off, nk * sizeof( unsigned ) ) );
+        get( ( void ** ) & mesh->d_sort_cnt, nk * sizeof( unsigned ) );
+        get( ( void ** ) & mesh->d_sort_off, nk * sizeof( unsigned ) );
         size_t tb = 0;
         KP_CUDA( cub::DeviceScan::ExclusiveSum( nullptr, tb, mesh->d_sort_cnt, mesh->d_sort_off,
                                                 ( int ) nk ) );
-        KP_CUDA( cudaMalloc( & mesh->d_sort_tmp, tb ) );
+        get( & mesh->d_sort_tmp, tb );
         mesh->sort_tmp_bytes = tb;
         mesh->sort_cells = nk;
     }
@@ -1456,7 +1461,7 @@ int * ensure_task_sort( kp_mesh_t * mesh, long long pq_cap )
         mesh->drop( mesh->d_sort_perm, mesh->perm_captured );
         mesh->d_sort_perm = nullptr;
         mesh->sort_perm = 0;
-        KP_CUDA( cudaMalloc( & mesh->d_sort_perm, n_slots * sizeof( int ) ) );
+        get( ( void ** ) & mesh->d_sort_perm, n_slots * sizeof( int ) );
         mesh->sort_perm = n_slots;
     }
     return mesh->d_sort_perm;
@@ -1479,15 +1484,16 @@ int * march_order( kp_mesh_t * mesh, long long n, cudaStream_t s )
         const relaxed_t relaxed;
         try
         {
-            return ensure_task_sort( mesh, mesh->pq_cap );
+            return ensure_task_sort( mesh, mesh->pq_cap, false );
         }
         catch( const error_t & )
         {
             cudaGetLastError(  );
+            if( ! mesh->sort_captured ) mesh->release_sort(  );
             return nullptr;
         }
     }
-    return ensure_task_sort( mesh, mesh->pq_cap );
+    return ensure_task_sort( mesh, mesh->pq_cap, true );
 }
 
 // Sorts the queued tasks by starting cell into P.pq_perm (k_task_sort).
@@ -1549,13 +1555,14 @@ void launch_peel_adjoint( const fwd_params_t & P, int tally_mode, int mode, cuda
 }
 
 template< int TALLY >
-void launch_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s )
+void launch_deferred( kp_mesh_t * mesh, fwd_params_t & P, cudaStream_t s )
 {
     mesh->tape_id = 0;                      // the queue is overwritten
     ensure_peel_queue( mesh, P.n_packets );
     const long long chunk = std::max< long long >( mesh->pq_cap / PQ_PER_PACKET, 1 );
-    ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
     int * perm = march_order( mesh, P.n_packets, s );
+    ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
+    begin_flux( mesh, TALLY, P, s );
     mesh->note_capture( s );
     static thread_local fwd_params_t C;
     for( long long done = 0; done < P.n_packets; done += chunk )
@@ -1570,7 +1577,7 @@ void launch_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s )
     }
 }
 
-void launch_deferred_solve( kp_mesh_t * mesh, const fwd_params_t & P, int tally_mode,
+void launch_deferred_solve( kp_mesh_t * mesh, fwd_params_t & P, int tally_mode,
                             cudaStream_t s )
 {
     if( tally_mode == KP_TALLY_FIXED ) launch_deferred< KP_TALLY_FIXED >( mesh, P, s );
@@ -1589,7 +1596,6 @@ extern "C" int kp_transport_forward( kp_mesh_t * mesh, const kp_transport_cfg_t 
         static thread_local kp::fwd_params_t P;
         kp::make_fwd_params( mesh, * cfg, * tallies, P );
         P.work = mesh->workspace(  );
-        kp::begin_flux( mesh, * tallies, cfg->tally_mode, P, ( cudaStream_t ) stream );
         if( cfg->image_n > 0 && P.n_packets > 0 )
         {   // peel-off rays through their own kernel
             if( cfg->tally_mode == KP_TALLY_FIXED )
@@ -1601,6 +1607,8 @@ extern "C" int kp_transport_forward( kp_mesh_t * mesh, const kp_transport_cfg_t 
         {
             auto s = ( cudaStream_t ) stream;
             kp::ensure_pool( mesh->pool, P.n_packets, s );
+            kp::begin_flux( mesh, cfg->tally_mode, P, s );
+            mesh->note_capture( s );
             KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
             kp::launch_walk( P, mesh->pool, cfg->tally_mode, kp::WALK_FORWARD, s );
             if( kp::split_event ) KP_CUDA( cudaEventRecord( kp::split_event, s ) );
@@ -1663,14 +1671,15 @@ namespace kp
 // chunks of the queue's capacity / 12, each walked and then marched, as
 // launch_deferred does for new packets alone.
 template< int TALLY >
-void launch_resume_deferred( kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s )
+void launch_resume_deferred( kp_mesh_t * mesh, fwd_params_t & P, cudaStream_t s )
 {
     const long long n_in = P.rs_n_in, items = n_in + P.n_packets;
     mesh->tape_id = 0;                      // the queue is overwritten
     ensure_peel_queue( mesh, items );
     const long long chunk = std::max< long long >( mesh->pq_cap / PQ_PER_PACKET, 1 );
-    ensure_pool( mesh->pool, std::min( chunk, items ), s );
     int * perm = march_order( mesh, items, s );
+    ensure_pool( mesh->pool, std::min( chunk, items ), s );
+    begin_flux( mesh, TALLY, P, s );
     mesh->note_capture( s );
     static thread_local fwd_params_t C;
     for( long long lo = 0; lo < items; lo += chunk )
@@ -1723,7 +1732,6 @@ extern "C" int kp_transport_forward_resume( kp_mesh_t * mesh, const kp_transport
         cudaStream_t s = ( cudaStream_t ) stream;
         if( P.n_packets + P.rs_n_in > 0 )
         {
-            kp::begin_flux( mesh, * tallies, cfg->tally_mode, P, s );
             const bool fx = cfg->tally_mode == KP_TALLY_FIXED;
             if( cfg->image_n > 0 )
             {
@@ -1733,6 +1741,8 @@ extern "C" int kp_transport_forward_resume( kp_mesh_t * mesh, const kp_transport
             else
             {
                 kp::ensure_pool( mesh->pool, P.n_packets + P.rs_n_in, s );
+                kp::begin_flux( mesh, cfg->tally_mode, P, s );
+                mesh->note_capture( s );
                 KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
                 kp::launch_walk( P, mesh->pool, cfg->tally_mode, kp::WALK_FORWARD, s );
                 if( kp::split_event ) KP_CUDA( cudaEventRecord( kp::split_event, s ) );

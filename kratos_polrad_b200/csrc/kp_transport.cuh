@@ -1102,14 +1102,14 @@ void task_sort( const kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s )
 template< int TALLY, bool TAPE >
 void launch_deferred_chunk( fwd_params_t & P, cudaStream_t s, kp_mesh_t * mesh );
 // A forward solve with its peel-off rays queued for k_peel, in chunks (no tape).
-void launch_deferred_solve( kp_mesh_t * mesh, const fwd_params_t & P, int tally_mode,
+void launch_deferred_solve( kp_mesh_t * mesh, fwd_params_t & P, int tally_mode,
                             cudaStream_t s );
 void launch_forward( const fwd_params_t & P, int tally_mode, cudaStream_t s );
 // The walk of one launch (k_walk): its kernel by P's queue, links, flux and
 // resume fields.  P.work, its packet counter, is zeroed by the caller.
 // Sums a float solve's flux in double, in the mesh's own array (P.flux_sum),
 // and adds the sums into the tally at its end.
-void begin_flux( kp_mesh_t * mesh, const kp_tallies_t & t, int tally_mode, fwd_params_t & P, cudaStream_t s );
+void begin_flux( kp_mesh_t * mesh, int tally_mode, fwd_params_t & P, cudaStream_t s );
 void fold_flux( const fwd_params_t & P, cudaStream_t s );
 enum walk_kind { WALK_FORWARD = 0, WALK_ADJ0 = 1, WALK_ADJ1 = 2 };
 struct walk_shape_t

@@ -315,6 +315,64 @@ void other_capture(  )
         kp_mesh_destroy( m );
     }
 }
+// A solve that fits the device without what is kept for speed alone (packet
+// pools, flux sums, the order by packet count) runs, whatever came before it.
+void short_memory(  )
+{
+    constexpr size_t SLACK = 1 << 16;                // a block's packets
+    for( int kind = 0; kind < 4; ++ kind )           // as queued, by cell, adjoint, tape
+    {
+        auto order = [ & ]( kp_mesh_t * m ) { if( kind == 1 ) kp_mesh_peel_order( m, KP_PEEL_ORDER_CELL ); };
+        auto solve = [ & ]( kp_mesh_t * m )
+        {
+            solve_t s( 100000, true );
+            if( kind < 2 ) s.flux( 64 * 64 * 64 );
+            return kind == 2 ? s.adjoint( m, nullptr ) : kind == 3 ? ( s.tape( m ), ( int ) KP_OK ) : s.run( m );
+        };
+        kp_mesh_t * m = make_mesh( 64 );
+        order( m );
+        expect( solve( m ) == KP_OK, "solve" );
+        const size_t need = F.used - m->pool.bytes - ( m->d_flux ? 64 * 64 * 64 * 8 : 0 );
+        kp_mesh_destroy( m );
+        for( int before = 0; before < 2; ++ before )
+        {
+            m = make_mesh( 64 );
+            order( m );
+            if( before )
+            {   // a pool, flux sums and a small queue of earlier solves
+                solve_t a( 50000, false ), b( 100, true );
+                expect( a.flux( 64 * 64 * 64 ).run( m ) == KP_OK && b.run( m ) == KP_OK, "earlier solves" );
+            }
+            F.limit = need + SLACK;
+            F.launches.clear(  );
+            expect( solve( m ) == KP_OK, "a solve that fits" );
+            for( const auto & l : F.launches )
+                if( l.kernel.find( "k_walk" ) != std::string::npos )
+                    expect( owner( ( uintptr_t ) l.P.pool ) && ( ! l.P.flux_sum || owner( ( uintptr_t ) l.P.flux_sum ) ),
+                            "the walk's memory" );
+            F.limit = ~ ( size_t ) 0;
+            F.last = cudaSuccess;
+            kp_mesh_destroy( m );
+            expect( F.live.empty(  ), "memory left behind" );
+        }
+    }
+    // an order by the packet count that a capture was given, and no memory for
+    // a larger solve's: that one marches as queued, the capture keeps its own
+    const cudaStream_t S = ( cudaStream_t ) 64;
+    kp_mesh_t * m = make_mesh( 160 );
+    solve_t s( 500000, true ), larger( 600000, true );
+    expect( s.run( m, S ) == KP_OK, "solve" );
+    F.capturing = S;
+    F.launches.clear(  );
+    expect( s.run( m, S ) == KP_OK && ! F.broken, "captured solve" );
+    F.capturing = nullptr;
+    const auto held = given(  );
+    F.limit = F.used + 600000ull * 12 * 64 + SLACK;
+    expect( larger.run( m, S ) == KP_OK, "larger solve" );
+    for( uintptr_t a : held )
+        expect( F.live.count( a ) != 0, "a captured order was freed" );
+    kp_mesh_destroy( m );
+}
 }   // namespace
 
 int main( int argc, char ** argv )
@@ -324,6 +382,7 @@ int main( int argc, char ** argv )
     else if( what == "tape_pool" ) tape_pool(  );
     else if( what == "captured" ) captured(  );
     else if( what == "other_capture" ) other_capture(  );
+    else if( what == "short_memory" ) short_memory(  );
     else return 2;
     if( fails == 0 ) std::printf( "OK %s\n", what.c_str(  ) );
     return fails != 0;
