@@ -93,6 +93,33 @@ struct alignas( 16 ) blk_meta_t
 };
 static_assert( sizeof( blk_meta_t ) == 16, "meta record" );
 
+// A launch's n items in shares, one per warp: the pieces w, w + n_warps, ... of
+// 2^unit items each.  Item `at` of warp w's share, at < size( w ), is item( w,
+// at ), which may lie past n in the last piece.
+struct share_t
+{
+    long long n, n_warps;
+    int       unit;
+
+    __host__ __device__ long long size( long long w ) const
+    {
+        const long long pieces = ( n + ( 1ll << unit ) - 1 ) >> unit;
+        return w < pieces ? ( ( pieces - w + n_warps - 1 ) / n_warps ) << unit : 0;
+    }
+    __host__ __device__ long long item( long long w, long long at ) const
+    {
+        return ( ( ( at >> unit ) * n_warps + w ) << unit ) + ( at & ( ( 1ll << unit ) - 1 ) );
+    }
+    // Pieces of at most 2^max_unit items, at least 16 of them to a share (so
+    // that a share is at most 1/16 longer than another).
+    static share_t make( long long n, long long n_warps, int max_unit )
+    {
+        int u = 0;
+        while( u < max_unit && n >= n_warps << ( u + 5 ) ) ++ u;
+        return share_t { n, n_warps, u };
+    }
+};
+
 // Whether stream s is being captured.
 inline bool capturing( cudaStream_t s )
 {

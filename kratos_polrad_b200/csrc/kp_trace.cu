@@ -363,6 +363,10 @@ __device__ __forceinline__ unsigned long long fx_round( double v )
 #define KP_TRACE_HOP 6               // lanes that wait for a block hand-off (4 and 10: 2%
                                      // slower in float, 4: 2% faster in double)
 #endif
+#ifndef KP_TRACE_UNIT
+#define KP_TRACE_UNIT 4              // log2 of the packets of a piece of a share (2: 1%
+                                     // slower in float, 3%, 5: as fast)
+#endif
 #ifndef KP_TRACE_ROUND
 #define KP_TRACE_ROUND 8             // segments per scheduling round (4: 1%, 16: 9% slower)
 #endif
@@ -377,7 +381,11 @@ constexpr int TRACE_THREADS = 128, TRACE_WARPS = TRACE_THREADS / 32;
 // The walk of a pool.  Each warp takes an even share of the packets and its
 // lanes the next of the share as they fall idle; block hand-offs wait for a
 // batch.  (Shares, not a common counter: calls on several streams share no
-// memory.)  What bounded one thread per packet was issue (71%) with 9 to 11
+// memory.)  A share is in small pieces from all over the pool: in one piece, the
+// live packets of a pool that is partly empty, or the long-lived ones, were a
+// few warps' where they lay together (2^20 slots, float, the first eighth live:
+// 0.96 ms, in pieces 0.39, a thread per packet 0.47; an eighth with 400 steps
+// and the rest with 2: 0.96, 0.41 and 0.53).  What bounded one thread per packet was issue (71%) with 9 to 11
 // lanes to an instruction and 214 to 270 instructions to a segment: four
 // divisions, the block's record read every step, and lanes waiting for the
 // longest packet and for single hand-offs.  With shares, quotients from
@@ -388,7 +396,7 @@ constexpr int TRACE_THREADS = 128, TRACE_WARPS = TRACE_THREADS / 32;
 // every step ends with par_base_t::regulate's test (particle_base.h:37-56).
 template< class f_t, int FLUX, bool PER >
 __global__ void __launch_bounds__( TRACE_THREADS, sizeof( f_t ) == 4 ? KP_TRACE_MINB : KP_TRACE_MINB_D )
-k_trace( const __grid_constant__ mesh_view_t m, long long n, f_t * __restrict__ xs,
+k_trace( const __grid_constant__ mesh_view_t m, const share_t share, f_t * __restrict__ xs,
          const f_t * __restrict__ dirs, int * __restrict__ cells,
          int * __restrict__ ibs, const f_t * __restrict__ propers,
          int * __restrict__ steps, int8_t * __restrict__ todos,
@@ -396,10 +404,9 @@ k_trace( const __grid_constant__ mesh_view_t m, long long n, f_t * __restrict__ 
 {
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u, below = ( 1u << lane ) - 1u;
-    const long long n_warps = ( long long ) gridDim.x * TRACE_WARPS;
     const long long w = ( long long ) blockIdx.x * TRACE_WARPS + ( threadIdx.x >> 5 );
-    long long next = n / n_warps * w + min( w, n % n_warps );            // this warp's share
-    const long long last = next + n / n_warps + ( w < n % n_warps ? 1 : 0 );
+    long long next = 0;
+    const long long last = share.size( w );
     const int nc0 = m.nc[ 0 ], nc1 = m.nc[ 1 ], nc2 = m.nc[ 2 ];
     enum { IDLE, SEGMENT, HOP };
     int phase = IDLE;
@@ -475,11 +482,12 @@ k_trace( const __grid_constant__ mesh_view_t m, long long n, f_t * __restrict__ 
                 todos[ p ] = TO_RM;
                 p = -1;
             }
-            const long long k = next + __popc( m_idle & below );
+            const long long at = next + __popc( m_idle & below );
+            const long long k = share.item( w, at );
             next = min( next + n_idle, last );
             // integrate::base_t::operator() only walks to_keep packets
             // (integrator.h:90-92)
-            if( phase == IDLE && k < last && todos[ k ] == TO_KEEP )
+            if( phase == IDLE && at < last && k < share.n && todos[ k ] == TO_KEEP )
             {
                 ib = ibs[ k ];
                 bool plain = true;
@@ -656,8 +664,9 @@ void launch_trace_k( const mesh_view_t & m, long long n, void * x, const void * 
     KP_CUDA( cudaDeviceGetAttribute( & n_sm, cudaDevAttrMultiProcessorCount, dev ) );
     KP_CUDA( cudaOccupancyMaxActiveBlocksPerMultiprocessor( & per_sm, k, TRACE_THREADS, 0 ) );
     const long long warps = std::min< long long >( ( long long ) n_sm * std::max( per_sm, 1 ) * TRACE_WARPS, n );
-    k<<< ( unsigned ) ( ( warps + TRACE_WARPS - 1 ) / TRACE_WARPS ), TRACE_THREADS, 0, s >>>(
-        m, n, ( f_t * ) x, ( const f_t * ) dir, cell, ib, ( const f_t * ) proper, step, todo, flux, fx_scale );
+    const long long grid = ( warps + TRACE_WARPS - 1 ) / TRACE_WARPS;
+    k<<< ( unsigned ) grid, TRACE_THREADS, 0, s >>>(
+        m, share_t::make( n, grid * TRACE_WARPS, KP_TRACE_UNIT ), ( f_t * ) x, ( const f_t * ) dir, cell, ib, ( const f_t * ) proper, step, todo, flux, fx_scale );
     KP_CUDA( cudaGetLastError(  ) );
 }
 

@@ -373,6 +373,34 @@ void short_memory(  )
         expect( F.live.count( a ) != 0, "a captured order was freed" );
     kp_mesh_destroy( m );
 }
+// A trace's shares hold every packet once, and packets that lie together in
+// the pool are many warps'.
+void shares(  )
+{
+    for( const long long w : { 4ll, 2960ll, 3552ll } )
+        for( const long long n : { 1ll, 31ll, 2001ll, 47359ll, 47360ll, 100003ll, 300001ll, 1048576ll } )
+        {
+            const kp::share_t s = kp::share_t::make( n, w, 4 );
+            std::vector< char > seen( n );
+            long long longest = 0, front = 0;        // of a share, and of its packets in the first eighth
+            for( long long k = 0; k < w; ++ k )
+            {
+                long long of_front = 0;
+                for( long long at = 0; at < s.size( k ); ++ at )
+                    if( const long long i = s.item( k, at ); i < n )
+                    {
+                        expect( ! seen[ i ], "a packet of two shares" );
+                        seen[ i ] = 1;
+                        of_front += i < n / 8;
+                    }
+                longest = std::max( longest, s.size( k ) );
+                front = std::max( front, of_front );
+            }
+            for( char c : seen ) if( ! c ) { expect( false, "a packet of no share" ); break; }
+            expect( longest <= n / w + n / w / 16 + 2, "an even share" );
+            expect( front <= n / 8 / w + ( 1 << s.unit ), "the pool's front in few shares" );
+        }
+}
 }   // namespace
 
 int main( int argc, char ** argv )
@@ -383,6 +411,7 @@ int main( int argc, char ** argv )
     else if( what == "captured" ) captured(  );
     else if( what == "other_capture" ) other_capture(  );
     else if( what == "short_memory" ) short_memory(  );
+    else if( what == "shares" ) shares(  );
     else return 2;
     if( fails == 0 ) std::printf( "OK %s\n", what.c_str(  ) );
     return fails != 0;

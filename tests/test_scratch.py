@@ -1,5 +1,5 @@
-"""The device memory that a mesh keeps for its solves (queues, packet pools,
-sums), followed without a GPU: tests/cpp/scratch_check.cu, linked with the
+"""The library's host code without a GPU, above all the device memory that a mesh
+keeps for its solves (queues, packet pools, sums): tests/cpp/scratch_check.cu, linked with the
 library's objects in place of the CUDA runtime, runs the entry points and looks
 at what they allocate, free and launch."""
 import glob
@@ -36,7 +36,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["host_mesh", "tape_pool", "captured", "other_capture", "short_memory"])
+@pytest.mark.parametrize("what", ["host_mesh", "tape_pool", "captured", "other_capture", "short_memory", "shares"])
 def test_scratch(program, what):
     r = subprocess.run([program, what], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == f"OK {what}\n", r.stdout + r.stderr
