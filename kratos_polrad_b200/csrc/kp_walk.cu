@@ -297,10 +297,11 @@ k_walk( const __grid_constant__ fwd_params_t P )
         }
     };
 
-    for( ;; )
+    for( bool start = true; ; start = false )
     {
-        // ---- births: whole batches, or what there is when nothing is ready ----
-        while( n_dead >= 32 || ( n_dead > 0 && n_ready == 0 && n_ev == 0 ) )
+        // ---- births: the whole pool at the start, then whole batches, or what
+        // there is when nothing is ready ----
+        while( n_dead >= 32 || ( n_dead > 0 && ( start || ( n_ready == 0 && n_ev == 0 ) ) ) )
         {
             const int take = min( n_dead, 32 );
             const bool act = ( int ) lane < take;

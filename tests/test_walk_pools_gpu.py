@@ -93,3 +93,13 @@ def test_full_pools_gradients(name):
     for x, y, z in zip(tape, whole, small):
         assert z.abs().sum() > 0
         assert torch.equal(x, z) and torch.equal(y, z)
+
+
+@pytest.mark.parametrize("n", [95_003, 120_001, 186_000])
+@pytest.mark.parametrize("name", ["slab", "amr_point"])
+def test_pools_of_no_whole_batch(name, n):
+    """Pools of 33 to 63 packets: a whole batch and a part of one are born at
+    the start."""
+    mesh, t = _solve_case(name, n_packets=n, max_scatter=30)
+    _same(forward(mesh, t), _single_kernel(mesh, t))
+    assert mesh.status() == 0
