@@ -385,7 +385,13 @@ typedef struct kp_tallies
  * rays (default 2^27, 8.6 GB); later solves reuse it, and the mesh frees it
  * with the mesh.  A solve that is captured into a graph needs a queue that is
  * large enough already; what it was given stays allocated until the mesh goes,
- * also where a later solve outgrows it. */
+ * also where a later solve outgrows it.  Further device memory, all of which
+ * yields to the queue where there is too little: the packets of the walk, up
+ * to 48 MB (on 148 SMs), lent to a solve by the process, which has as many such
+ * pools as solves were in flight at once and frees all but one when a mesh or
+ * a batch goes (a captured solve's pool is its mesh's, kept with it); a float
+ * flux with a carry, 8 B per cell of the mesh, kept with it; and the march
+ * order (kp_mesh_peel_order). */
 int kp_transport_forward( kp_mesh_t * mesh, const kp_transport_cfg_t * cfg,
                           const kp_tallies_t * tallies, void * stream );
 

@@ -558,7 +558,7 @@ void adjoint_params( kp_mesh_t * mesh, const kp_transport_cfg_t * cfg, const flo
 // The adjoint once every queued ray of the chunk C has its score in adj_G:
 // R per packet, the second replay, the deposits along the rays, and the
 // packets left to k_adjoint (whose first replay counts nothing).
-void adjoint_second_half( kp::fwd_params_t & C, kp::pool_mem_t & pool, int tally_mode, cudaStream_t s )
+void adjoint_second_half( kp::fwd_params_t & C, const kp::walk_pool_t & pool, int tally_mode, cudaStream_t s )
 {
     const bool fx = tally_mode == KP_TALLY_FIXED;
     const int threads = kp::FWD_THREADS;
@@ -630,7 +630,7 @@ extern "C" int kp_transport_adjoint( kp_mesh_t * mesh, const kp_transport_cfg_t 
         kp::adjoint_buffers( mesh, P, std::min( chunk, P.n_packets ) );
         // both marches read the queue in the forward solve's order
         int * perm = kp::march_order( mesh, P.n_packets, s );
-        kp::ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
+        const kp::walk_pool_t pool( mesh->pool, std::min( chunk, P.n_packets ), s );
         mesh->note_capture( s );
         static thread_local kp::fwd_params_t C;
         for( long long done = 0; done < P.n_packets; done += chunk )
@@ -643,10 +643,10 @@ extern "C" int kp_transport_adjoint( kp_mesh_t * mesh, const kp_transport_cfg_t 
             KP_CUDA( cudaMemsetAsync( C.adj_head, 0xff, C.n_packets * sizeof( int ), s ) );
             KP_CUDA( cudaMemsetAsync( C.adj_flag, 0, C.n_packets * sizeof( int ), s ) );
             // first replay: walks, vertex rays queued
-            kp::launch_walk( C, mesh->pool, cfg->tally_mode, kp::WALK_ADJ0, s );
+            kp::launch_walk( C, pool, cfg->tally_mode, kp::WALK_ADJ0, s );
             if( perm ) kp::task_sort( mesh, C, s );                     // by starting cell
             kp::launch_peel_adjoint( C, cfg->tally_mode, 1, s );       // scores G
-            adjoint_second_half( C, mesh->pool, cfg->tally_mode, s );
+            adjoint_second_half( C, pool, cfg->tally_mode, s );
         }
     } );
 }
@@ -682,16 +682,16 @@ extern "C" int kp_transport_forward_tape( kp_mesh_t * mesh, const kp_transport_c
         P.pq_perm = kp::march_order( mesh, P.n_packets, ( cudaStream_t ) stream );
         const bool sorted = P.pq_perm != nullptr;
         auto s = ( cudaStream_t ) stream;
-        kp::ensure_pool( mesh->pool, P.n_packets, s );
+        const kp::walk_pool_t pool( mesh->pool, P.n_packets, s );
         kp::begin_flux( mesh, cfg->tally_mode, P, s );
         mesh->note_capture( s );
         KP_CUDA( cudaMemsetAsync( P.work, 0, 4 * sizeof( unsigned long long ), s ) );
         KP_CUDA( cudaMemsetAsync( P.adj_head, 0xff, P.n_packets * sizeof( int ), s ) );
         KP_CUDA( cudaMemsetAsync( P.adj_flag, 0, P.n_packets * sizeof( int ), s ) );
         if( cfg->tally_mode == KP_TALLY_FIXED )
-            kp::launch_deferred_chunk< KP_TALLY_FIXED, true >( P, s, mesh );
+            kp::launch_deferred_chunk< KP_TALLY_FIXED, true >( P, s, mesh, pool );
         else
-            kp::launch_deferred_chunk< KP_TALLY_FLOAT, true >( P, s, mesh );
+            kp::launch_deferred_chunk< KP_TALLY_FLOAT, true >( P, s, mesh, pool );
         kp::fold_flux( P, s );
         kp::fold_carry( * cfg, * tallies, s );
         mesh->tape_cfg = * cfg;
@@ -722,15 +722,13 @@ extern "C" int kp_transport_adjoint_tape( kp_mesh_t * mesh, long long tape_id,
         kp::adjoint_buffers( mesh, P, mesh->tape_n );      // the taped solve's layout
         P.pq_perm = mesh->tape_sorted ? mesh->d_sort_perm : nullptr;   // ... and order
         auto s = ( cudaStream_t ) stream;
-        // a solve without an image since then leaves the tape, but may have
-        // lost the pool for want of memory
-        kp::ensure_pool( mesh->pool, mesh->tape_n, s );
+        const kp::walk_pool_t pool( mesh->pool, mesh->tape_n, s );
         mesh->note_capture( s );
         mesh->refresh_ext( s );
         const unsigned gs = 4 * 148;
         kp::k_adj_score<<< gs, 256, 0, s >>>( P );                        // G from the tape
         KP_CUDA( cudaGetLastError(  ) );
-        adjoint_second_half( P, mesh->pool, cfg->tally_mode, s );
+        adjoint_second_half( P, pool, cfg->tally_mode, s );
     } );
 }
 

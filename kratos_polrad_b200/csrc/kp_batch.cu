@@ -38,7 +38,7 @@ struct kp_batch
     float      * d_ext = nullptr;              // sca + abs per cell, from d_sigma
     unsigned   * d_status = nullptr;
     unsigned long long * d_work = nullptr;
-    kp::pool_mem_t pool;                       // packets of the walk in progress
+    kp::pool_mem_t pool;                       // packets of its captured launch
     long long  * d_prefix = nullptr;
     long long  * d_prefix_trial = nullptr;      // autotuner sample
     kp::scene_dev_t * d_scenes = nullptr;
@@ -56,6 +56,7 @@ struct kp_batch
         cudaFree( d_ext );
         cudaFree( d_status ); cudaFree( d_work ); cudaFree( d_prefix );
         cudaFree( d_prefix_trial ); cudaFree( d_scenes );
+        kp::trim_pools( false, true );
     }
 };
 
@@ -101,8 +102,9 @@ void make_batch_params( kp_batch_t * b, const kp_transport_cfg_t & c, void * mu,
 
 void launch( kp_batch_t * b, kp::fwd_params_t & P, int tally_mode, cudaStream_t s )
 {
+    const kp::walk_pool_t pool( b->pool, P.n_packets, s );
     KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
-    kp::launch_walk( P, b->pool, tally_mode, kp::WALK_FORWARD, s, b->grid_pct );
+    kp::launch_walk( P, pool, tally_mode, kp::WALK_FORWARD, s, b->grid_pct );
 }
 
 }   // namespace
@@ -200,7 +202,6 @@ int kp_batch_create( int n_scenes, const kp_scene_t * sc, kp_batch_t ** out )
                              cudaMemcpyHostToDevice ) );
         KP_CUDA( cudaMemcpy( b->d_scenes, b->scenes.data(  ),
                              b->scenes.size(  ) * sizeof( kp::scene_dev_t ), cudaMemcpyHostToDevice ) );
-        kp::ensure_pool( b->pool, b->total, nullptr );
         copy_sigma( b.get(  ), nullptr );
         KP_CUDA( cudaDeviceSynchronize(  ) );
         auto & v = b->view;

@@ -140,13 +140,14 @@ struct relaxed_t
     relaxed_t & operator=( const relaxed_t & ) = delete;
 };
 
-// Device memory of the walk's packet pools (kp_walk.cu).
+// Device memory of the packet pools of an owner's captured solves (kp_walk.cu):
+// a capture keeps its pool's address until the owner goes.
 struct pool_mem_t
 {
     void * d = nullptr;
     size_t bytes = 0;
-    void * old = nullptr;                 // an outgrown pool that a captured launch uses
-    bool   captured = false, full = false;     // d is in a captured launch; of the full size
+    void * old = nullptr;                 // an outgrown pool of an earlier capture
+    bool   full = false;                  // d has the full size
 
     pool_mem_t(  ) = default;
     pool_mem_t( const pool_mem_t & ) = delete;
@@ -158,9 +159,29 @@ struct pool_mem_t
         if( old ) cudaFree( old );
         d = old = nullptr;
         bytes = 0;
-        captured = full = false;
+        full = false;
     }
 };
+
+// The packet pools of one solve of `items` packets on stream s: its owner's when
+// s is being captured, else lent to it until this goes (kp_walk.cu).
+class walk_pool_t
+{
+public:
+    walk_pool_t( pool_mem_t & own, long long items, cudaStream_t s );
+    ~ walk_pool_t(  );
+    walk_pool_t( const walk_pool_t & ) = delete;
+    walk_pool_t & operator=( const walk_pool_t & ) = delete;
+    void * d = nullptr;
+    size_t bytes = 0;
+private:
+    cudaStream_t stream;
+    void * lent = nullptr;
+};
+// Frees what is there to be lent on the current device and is not in use: all of
+// it (in_flight: also what a stream may still use; the free waits for that), or
+// all but one (keep).
+void trim_pools( bool in_flight, bool keep );
 
 struct mesh_view_t
 {
@@ -234,7 +255,7 @@ struct kp_mesh
     float      * d_vol_f = nullptr;  double * d_vol_d = nullptr;
 
     unsigned long long * d_work = nullptr;   // scratch: packet counters
-    kp::pool_mem_t pool;                     // packets of the walk in progress
+    kp::pool_mem_t pool;                     // packets of its captured solves
     double     * d_flux = nullptr;           // a float solve's flux sums, one per cell
 
     kp::mesh_view_t view(  ) const;
@@ -249,7 +270,7 @@ struct kp_mesh
     // other marks the buffers that a solve on s was given, if s is captured.
     void drop( void * p, bool & was_captured );
     // Memory that a solve cannot do without.  Where there is too little, the
-    // mesh first gives back what it keeps for speed alone: the packet pool, the
+    // mesh first gives back what is kept for speed alone: the packet pools, the
     // flux sums and an order that only the packet count asked for.  A solve
     // makes those last, as large as still fits.
     void need( void ** p, size_t bytes );

@@ -190,7 +190,7 @@ void kp_mesh::need( void ** p, size_t bytes )
     if( e == cudaErrorMemoryAllocation )
     {
         cudaGetLastError(  );
-        if( ! pool.captured ) pool.release(  );
+        kp::trim_pools( true, false );
         if( ! sort_captured )
         {
             cudaFree( d_flux );
@@ -231,6 +231,7 @@ void kp_mesh::release(  )
     cudaFree( d_status ); d_status = nullptr;
     cudaFree( d_work );   d_work   = nullptr;
     pool.release(  );
+    kp::trim_pools( false, true );
     cudaFree( d_flux );   d_flux   = nullptr;
     cudaFree( d_pq );     d_pq     = nullptr; pq_cap = 0;
     release_sort(  );

@@ -1531,18 +1531,20 @@ void launch_peel( const fwd_params_t & P, cudaStream_t s )
 }
 
 template< int TALLY, bool TAPE >
-void launch_deferred_chunk( fwd_params_t & P, cudaStream_t s, kp_mesh_t * mesh )
+void launch_deferred_chunk( fwd_params_t & P, cudaStream_t s, kp_mesh_t * mesh, const walk_pool_t & pool )
 {
     P.pq_count = P.work + 1;
     P.pq_next = P.work + 2;
     KP_CUDA( cudaMemsetAsync( P.work, 0, 3 * sizeof( unsigned long long ), s ) );
-    launch_walk( P, mesh->pool, TALLY, WALK_FORWARD, s );
+    launch_walk( P, pool, TALLY, WALK_FORWARD, s );
     if( split_event ) KP_CUDA( cudaEventRecord( split_event, s ) );
     if( P.pq_perm ) task_sort( mesh, P, s );
     launch_peel< TALLY, TAPE ? 3 : 0 >( P, s );
 }
-template void launch_deferred_chunk< KP_TALLY_FIXED, true >( fwd_params_t &, cudaStream_t, kp_mesh_t * );
-template void launch_deferred_chunk< KP_TALLY_FLOAT, true >( fwd_params_t &, cudaStream_t, kp_mesh_t * );
+template void launch_deferred_chunk< KP_TALLY_FIXED, true >( fwd_params_t &, cudaStream_t, kp_mesh_t *,
+                                                              const walk_pool_t & );
+template void launch_deferred_chunk< KP_TALLY_FLOAT, true >( fwd_params_t &, cudaStream_t, kp_mesh_t *,
+                                                              const walk_pool_t & );
 
 // The deferred adjoint's marches of the queued vertex rays: mode 1 measures
 // their scores, mode 2 deposits along them (k_peel).
@@ -1561,7 +1563,7 @@ void launch_deferred( kp_mesh_t * mesh, fwd_params_t & P, cudaStream_t s )
     ensure_peel_queue( mesh, P.n_packets );
     const long long chunk = std::max< long long >( mesh->pq_cap / PQ_PER_PACKET, 1 );
     int * perm = march_order( mesh, P.n_packets, s );
-    ensure_pool( mesh->pool, std::min( chunk, P.n_packets ), s );
+    const walk_pool_t pool( mesh->pool, std::min( chunk, P.n_packets ), s );
     begin_flux( mesh, TALLY, P, s );
     mesh->note_capture( s );
     static thread_local fwd_params_t C;
@@ -1573,7 +1575,7 @@ void launch_deferred( kp_mesh_t * mesh, fwd_params_t & P, cudaStream_t s )
         C.pq_perm = perm;
         C.pid0 = P.pid0 + done;
         C.n_packets = std::min( chunk, P.n_packets - done );
-        launch_deferred_chunk< TALLY, false >( C, s, mesh );
+        launch_deferred_chunk< TALLY, false >( C, s, mesh, pool );
     }
 }
 
@@ -1606,11 +1608,11 @@ extern "C" int kp_transport_forward( kp_mesh_t * mesh, const kp_transport_cfg_t 
         else
         {
             auto s = ( cudaStream_t ) stream;
-            kp::ensure_pool( mesh->pool, P.n_packets, s );
+            const kp::walk_pool_t pool( mesh->pool, P.n_packets, s );
             kp::begin_flux( mesh, cfg->tally_mode, P, s );
             mesh->note_capture( s );
             KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
-            kp::launch_walk( P, mesh->pool, cfg->tally_mode, kp::WALK_FORWARD, s );
+            kp::launch_walk( P, pool, cfg->tally_mode, kp::WALK_FORWARD, s );
             if( kp::split_event ) KP_CUDA( cudaEventRecord( kp::split_event, s ) );
         }
         kp::fold_flux( P, ( cudaStream_t ) stream );
@@ -1678,7 +1680,7 @@ void launch_resume_deferred( kp_mesh_t * mesh, fwd_params_t & P, cudaStream_t s 
     ensure_peel_queue( mesh, items );
     const long long chunk = std::max< long long >( mesh->pq_cap / PQ_PER_PACKET, 1 );
     int * perm = march_order( mesh, items, s );
-    ensure_pool( mesh->pool, std::min( chunk, items ), s );
+    const walk_pool_t pool( mesh->pool, std::min( chunk, items ), s );
     begin_flux( mesh, TALLY, P, s );
     mesh->note_capture( s );
     static thread_local fwd_params_t C;
@@ -1694,7 +1696,7 @@ void launch_resume_deferred( kp_mesh_t * mesh, fwd_params_t & P, cudaStream_t s 
         const long long first = std::max( lo, n_in );   // first new packet's item
         C.pid0 = P.pid0 + ( first - n_in );
         C.n_packets = std::max< long long >( hi - first, 0 );
-        launch_deferred_chunk< TALLY, false >( C, s, mesh );
+        launch_deferred_chunk< TALLY, false >( C, s, mesh, pool );
     }
 }
 }   // namespace kp
@@ -1740,11 +1742,11 @@ extern "C" int kp_transport_forward_resume( kp_mesh_t * mesh, const kp_transport
             }
             else
             {
-                kp::ensure_pool( mesh->pool, P.n_packets + P.rs_n_in, s );
+                const kp::walk_pool_t pool( mesh->pool, P.n_packets + P.rs_n_in, s );
                 kp::begin_flux( mesh, cfg->tally_mode, P, s );
                 mesh->note_capture( s );
                 KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
-                kp::launch_walk( P, mesh->pool, cfg->tally_mode, kp::WALK_FORWARD, s );
+                kp::launch_walk( P, pool, cfg->tally_mode, kp::WALK_FORWARD, s );
                 if( kp::split_event ) KP_CUDA( cudaEventRecord( kp::split_event, s ) );
             }
             kp::fold_flux( P, s );

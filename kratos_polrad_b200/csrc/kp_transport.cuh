@@ -1100,13 +1100,11 @@ void task_sort( const kp_mesh_t * mesh, const fwd_params_t & P, cudaStream_t s )
 // The walk of one chunk, then the march of its queue (in P.pq_perm's order
 // when set, sorted first with the mesh's buffers).
 template< int TALLY, bool TAPE >
-void launch_deferred_chunk( fwd_params_t & P, cudaStream_t s, kp_mesh_t * mesh );
+void launch_deferred_chunk( fwd_params_t & P, cudaStream_t s, kp_mesh_t * mesh, const walk_pool_t & pool );
 // A forward solve with its peel-off rays queued for k_peel, in chunks (no tape).
 void launch_deferred_solve( kp_mesh_t * mesh, fwd_params_t & P, int tally_mode,
                             cudaStream_t s );
 void launch_forward( const fwd_params_t & P, int tally_mode, cudaStream_t s );
-// The walk of one launch (k_walk): its kernel by P's queue, links, flux and
-// resume fields.  P.work, its packet counter, is zeroed by the caller.
 // Sums a float solve's flux in double, in the mesh's own array (P.flux_sum),
 // and adds the sums into the tally at its end.
 void begin_flux( kp_mesh_t * mesh, int tally_mode, fwd_params_t & P, cudaStream_t s );
@@ -1117,9 +1115,10 @@ struct walk_shape_t
     long long warps;
     int       per_warp;            // pool packets of a warp
 };
-walk_shape_t walk_shape( long long items, long long warps, const pool_mem_t & mem );
-void ensure_pool( pool_mem_t & mem, long long items, cudaStream_t s );
-void launch_walk( fwd_params_t & P, pool_mem_t & mem, int tally_mode, walk_kind kind, cudaStream_t s,
+walk_shape_t walk_shape( long long items, long long warps, const walk_pool_t & mem );
+// The walk of one launch (k_walk): its kernel by P's queue, links, flux and
+// resume fields.  P.work, its packet counter, is zeroed by the caller.
+void launch_walk( fwd_params_t & P, const walk_pool_t & mem, int tally_mode, walk_kind kind, cudaStream_t s,
                   int grid_pct = 100 );
 
 }   // namespace kp

@@ -33,6 +33,10 @@
 // 4.49 -> 3.86 ms.
 #include "kp_transport.cuh"
 
+#include <algorithm>
+#include <mutex>
+#include <vector>
+
 namespace kp
 {
 
@@ -792,7 +796,7 @@ k_walk( const __grid_constant__ fwd_params_t P )
 }
 
 template< int TALLY, int KIND, bool IMG, bool TAPE, bool FLUX, bool RESUME >
-void launch_walk_k( fwd_params_t & P, pool_mem_t & mem, cudaStream_t s, int pct )
+void launch_walk_k( fwd_params_t & P, const walk_pool_t & mem, cudaStream_t s, int pct )
 {
     const auto k = k_walk< TALLY, KIND, IMG, TAPE, FLUX, RESUME >;
     const long long items = P.n_packets + P.rs_n_in;
@@ -805,7 +809,7 @@ void launch_walk_k( fwd_params_t & P, pool_mem_t & mem, cudaStream_t s, int pct 
 }
 
 template< int TALLY >
-void launch_walk_t( fwd_params_t & P, pool_mem_t & mem, walk_kind kind, cudaStream_t s, int pct )
+void launch_walk_t( fwd_params_t & P, const walk_pool_t & mem, walk_kind kind, cudaStream_t s, int pct )
 {
     const bool img = P.pq != nullptr, fl = P.flux != nullptr, tape = P.pq_link != nullptr;
     if( kind == WALK_ADJ0 )      launch_walk_k< TALLY, WALK_ADJ0, true, true,  false, false >( P, mem, s, pct );
@@ -844,7 +848,7 @@ long long pool_size( long long items, long long warps )
 // holds `warps` warps, within the memory there is: at least a chunk for each
 // warp of a block, or the launch is refused (a warp without a pool would end
 // at once, and its packets with it).
-walk_shape_t walk_shape( long long items, long long warps, const pool_mem_t & mem )
+walk_shape_t walk_shape( long long items, long long warps, const walk_pool_t & mem )
 {
     const long long room = ( long long ) ( mem.bytes / sizeof( pool_chunk_t ) );    // chunks
     require( room >= WALK_WARPS, "no pool for the walk's packets", KP_ERR_ALLOC );
@@ -857,64 +861,172 @@ walk_shape_t walk_shape( long long items, long long warps, const pool_mem_t & me
     return walk_shape_t { warps, ( int ) per };
 }
 
-// Makes the pool large enough for a launch of `items` packets, at once where
-// a stream is being captured too.  A captured launch keeps its pool's address:
-// from then on a pool that is outgrown is kept (`old`) until its owner goes,
-// and the next one has the full size (48 MB on 148 SMs), so there is at most
-// one of these.  Where the memory is short, a smaller pool does.
-void ensure_pool( pool_mem_t & mem, long long items, cudaStream_t s )
+// Bytes of the pools of a launch of `items` packets (-1: of any launch, 48 MB on
+// 148 SMs) on the current device.
+static size_t pool_bytes( long long items )
 {
     int dev = 0, n_sm = 0;
     KP_CUDA( cudaGetDevice( & dev ) );
     KP_CUDA( cudaDeviceGetAttribute( & n_sm, cudaDevAttrMultiProcessorCount, dev ) );
-    const bool in_capture = capturing( s );
     const long long warps = ( long long ) n_sm * KP_WALK_MINB * WALK_WARPS;
-    auto bytes = [ & ]( long long n )
-    {
-        const long long used = ( std::min( warps, n ) + WALK_WARPS - 1 ) / WALK_WARPS * WALK_WARPS;
-        return ( size_t ) used * ( ( pool_size( n, warps ) + 31 ) / 32 ) * sizeof( pool_chunk_t );
-    };
-    size_t want = bytes( items );
-    if( mem.bytes < want && ! mem.full )
-    {
-        const relaxed_t relaxed;
-        void * d = nullptr;
-        const bool keep = mem.captured || ( in_capture && mem.d );
-        if( ! keep )
-        {
-            cudaFree( mem.d );
-            mem.d = nullptr;
-            mem.bytes = 0;
-        }
-        else
-            want = bytes( warps * KP_WALK_POOL );
-        cudaError_t e = cudaMalloc( & d, want );
-        const size_t least = std::max( mem.bytes, WALK_WARPS * sizeof( pool_chunk_t ) );
-        while( e == cudaErrorMemoryAllocation && want / 2 > least )
-        {
-            cudaGetLastError(  );
-            want /= 2;
-            e = cudaMalloc( & d, want );
-        }
-        if( e == cudaSuccess )
-        {
-            if( keep ) mem.old = mem.d;
-            mem.d = d;
-            mem.bytes = want;
-            mem.full = keep;
-        }
-        else if( mem.d )
-            cudaGetLastError(  );                 // the pool there is
-        else
-        {
-            cudaGetLastError(  );
-            KP_CUDA( e );
-        }
-    }
-    mem.captured = mem.captured || in_capture;
+    if( items < 0 ) items = warps * KP_WALK_POOL;
+    const long long used = ( std::min( warps, items ) + WALK_WARPS - 1 ) / WALK_WARPS * WALK_WARPS;
+    return ( size_t ) used * ( ( pool_size( items, warps ) + 31 ) / 32 ) * sizeof( pool_chunk_t );
 }
 
-void launch_walk( fwd_params_t & P, pool_mem_t & mem, int tally_mode, walk_kind kind, cudaStream_t s,
+// An allocation of `bytes`, where the memory is short of half as many, a quarter,
+// ..., down to a block's pools and to more than `least`; null if there is none.
+static void * alloc_pool( size_t & bytes, size_t least )
+{
+    void * d = nullptr;
+    least = std::max( least + 1, WALK_WARPS * sizeof( pool_chunk_t ) );
+    for( ; bytes >= least; bytes /= 2 )
+    {
+        const cudaError_t e = cudaMalloc( & d, bytes );
+        if( e == cudaSuccess ) return d;
+        cudaGetLastError(  );
+        if( e != cudaErrorMemoryAllocation ) KP_CUDA( e );
+    }
+    return nullptr;
+}
+
+// Pools that solves borrow, for the whole process.  An allocation takes 0.4 ms
+// whatever its size, as long as a small solve, so a pool per mesh (and 48 MB in
+// each) left a mesh's first solve slower than one without: 2000 packets without
+// an image 0.66 ms, 0.87 with it; 1e5 0.88 and 1.27.  A pool is free for a
+// solve on the stream that used it last (the solves are in that stream's order)
+// or once that use has ended; a solve that finds none makes one.  So there are at most as
+// many as solves were in flight at once, and all but one are freed when a mesh
+// or a batch goes.
+namespace
+{
+struct lent_t
+{
+    void * d;
+    size_t bytes;
+    int    device;
+    cudaEvent_t done;                     // of the last solve
+    unsigned long long stream;            // ... and its stream's id
+    bool   busy;                          // in the hands of a call under way
+};
+std::mutex lent_mutex;
+std::vector< lent_t * > & lent_pools(  )
+{
+    static auto * v = new std::vector< lent_t * >;   // the driver is gone before a static's end
+    return * v;
+}
+
+bool ended( const lent_t & l )
+{
+    const cudaError_t e = cudaEventQuery( l.done );
+    if( e != cudaSuccess ) cudaGetLastError(  );
+    return e == cudaSuccess;
+}
+
+lent_t * borrow( long long items, cudaStream_t s )
+{
+    const size_t want = pool_bytes( items );
+    int dev = 0;
+    unsigned long long id = 0;
+    KP_CUDA( cudaGetDevice( & dev ) );
+    KP_CUDA( cudaStreamGetId( s, & id ) );
+    const relaxed_t relaxed;
+    const std::lock_guard< std::mutex > lock( lent_mutex );
+    auto & pools = lent_pools(  );
+    lent_t * best = nullptr, * other = nullptr;      // free for s, in use on another stream
+    for( lent_t * l : pools )
+        if( ! l->busy && l->device == dev )
+        {
+            if( l->stream != id && ! ended( * l ) ) other = l;
+            else if( ! best || ( best->bytes < want && l->bytes > best->bytes ) ) best = l;
+        }
+    if( ! best || best->bytes < want )
+    {   // a full one, or, with little memory left, what is more than there is
+        size_t bytes = pool_bytes( -1 );
+        if( void * d = alloc_pool( bytes, best ? best->bytes : 0 ) )
+        {
+            best = new lent_t { d, bytes, dev, nullptr, id, false };
+            if( const cudaError_t e = cudaEventCreateWithFlags( & best->done, cudaEventDisableTiming ); e != cudaSuccess )
+            {
+                cudaFree( d );
+                delete best;
+                KP_CUDA( e );
+            }
+            pools.push_back( best );
+        }
+    }
+    if( ! best && other )
+    {   // no memory for another: after that stream's solve
+        KP_CUDA( cudaStreamWaitEvent( s, other->done, 0 ) );
+        best = other;
+    }
+    require( best != nullptr, "no memory for the walk's packets", KP_ERR_ALLOC );
+    best->stream = id;
+    best->busy = true;
+    return best;
+}
+}   // namespace
+
+void trim_pools( bool in_flight, bool keep )
+{
+    const std::lock_guard< std::mutex > lock( lent_mutex );
+    auto & pools = lent_pools(  );
+    int dev = 0;
+    if( pools.empty(  ) || cudaGetDevice( & dev ) != cudaSuccess ) return;
+    const relaxed_t relaxed;
+    for( size_t k = 0; k < pools.size(  ); )
+    {
+        lent_t * l = pools[ k ];
+        if( l->busy || l->device != dev || ! ( in_flight || ended( * l ) ) ) { ++ k; continue; }
+        if( keep ) { keep = false; ++ k; continue; }
+        cudaFree( l->d );
+        cudaEventDestroy( l->done );
+        delete l;
+        pools.erase( pools.begin(  ) + k );
+    }
+}
+
+// A captured solve takes its owner's pool, allocated in the capture when there is
+// none or it is too small.  One that is outgrown is kept (`old`) and the next has
+// the full size, so there is at most one of these.
+walk_pool_t::walk_pool_t( pool_mem_t & own, long long items, cudaStream_t s ) : stream( s )
+{
+    if( items <= 0 ) return;
+    if( ! capturing( s ) )
+    {
+        lent_t * l = borrow( items, s );
+        lent = l;
+        d = l->d;
+        bytes = l->bytes;
+        return;
+    }
+    size_t want = pool_bytes( own.d ? -1 : items );
+    if( own.bytes < pool_bytes( items ) && ! own.full )
+    {
+        const relaxed_t relaxed;
+        if( void * p = alloc_pool( want, own.bytes ) )
+        {
+            own.old = own.d;
+            own.full = own.d != nullptr;
+            own.d = p;
+            own.bytes = want;
+        }
+    }
+    d = own.d;
+    bytes = own.bytes;
+    require( d != nullptr, "no memory for the walk's packets", KP_ERR_ALLOC );
+}
+
+walk_pool_t::~ walk_pool_t(  )
+{
+    if( ! lent ) return;
+    auto * l = static_cast< lent_t * >( lent );
+    cudaEventRecord( l->done, stream );
+    const std::lock_guard< std::mutex > lock( lent_mutex );
+    l->busy = false;
+}
+
+void launch_walk( fwd_params_t & P, const walk_pool_t & mem, int tally_mode, walk_kind kind, cudaStream_t s,
                   int pct )
 {
     if( P.n_packets + P.rs_n_in == 0 ) return;
