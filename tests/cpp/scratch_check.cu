@@ -287,6 +287,32 @@ void captured(  )
         expect( F.live.size(  ) <= 1, "memory left behind" );     // a pool to be lent
     }
 }
+// Where the packet count chooses the march order, it does so at the stated count
+// and only where the caller left the choice.
+void order_by_count(  )
+{
+    kp_mesh_t * m = make_mesh( 160 );                // 16 MB of extinction
+    auto sorted = [ & ]( int order, long long n )
+    {
+        kp_mesh_peel_order( m, order );
+        F.launches.clear(  );
+        expect( solve_t( n, true ).run( m ) == KP_OK, "solve" );
+        int sorts = 0, marches = 0;
+        for( const auto & l : F.launches )
+        {
+            sorts += l.kernel.find( "k_task_sort" ) != std::string::npos;
+            marches += l.kernel.find( "k_peel" ) != std::string::npos && l.P.pq_perm != nullptr;
+        }
+        expect( sorts == 2 * marches, "sorted and marched so" );
+        return marches == 1;
+    };
+    expect( ! sorted( KP_PEEL_ORDER_AUTO, KP_PEEL_SORT_MANY - 1 ), "as queued below the count" );
+    expect( sorted( KP_PEEL_ORDER_AUTO, KP_PEEL_SORT_MANY ), "by cell from the count on" );
+    expect( ! sorted( KP_PEEL_ORDER_AUTO, 1000 ), "as queued again" );
+    expect( ! sorted( KP_PEEL_ORDER_QUEUE, KP_PEEL_SORT_MANY ) && sorted( KP_PEEL_ORDER_CELL, 1000 ), "the caller's order" );
+    kp_mesh_destroy( m );
+}
+
 // What a solve allocates beside its queue, for speed alone, disturbs no capture
 // under way in another thread, and a captured solve has it too.
 void other_capture(  )
@@ -456,6 +482,7 @@ int main( int argc, char ** argv )
     else if( what == "other_capture" ) other_capture(  );
     else if( what == "short_memory" ) short_memory(  );
     else if( what == "shares" ) shares(  );
+    else if( what == "order_by_count" ) order_by_count(  );
     else if( what == "first_solve" ) first_solve(  );
     else return 2;
     if( fails == 0 ) std::printf( "OK %s\n", what.c_str(  ) );

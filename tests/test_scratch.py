@@ -36,7 +36,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["host_mesh", "tape_pool", "captured", "other_capture", "short_memory", "shares", "first_solve"])
+@pytest.mark.parametrize("what", ["host_mesh", "tape_pool", "captured", "other_capture", "short_memory", "shares", "first_solve", "order_by_count"])
 def test_scratch(program, what):
     r = subprocess.run([program, what], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == f"OK {what}\n", r.stdout + r.stderr
