@@ -511,7 +511,7 @@ typedef struct kp_scene
 
 typedef struct kp_tune_result
 {
-    int       threads;         /* threads per block                            */
+    int       threads;         /* threads per block (128: not tuned)           */
     int       lane_batch;      /* event batch (see kp_transport_cfg_t)         */
     int       grid_pct;        /* persistent grid, percent of resident blocks  */
     float     sample_ms;       /* time of the best candidate on the sample     */
@@ -537,8 +537,9 @@ int kp_batch_forward( kp_batch_t * batch, const kp_transport_cfg_t * cfg, void *
  * (non-default), later calls replay it. */
 int kp_batch_graph_launch( kp_batch_t * batch, const kp_transport_cfg_t * cfg, void * mu,
                            unsigned long long * counters, void * stream );
-/* Autotuner: times candidate launch shapes (event batch, grid fill) on `fraction` of every scene's packets, tallying into
- * mu_scratch (same shape as mu), and keeps the fastest for later launches. */
+/* Autotuner: times candidate launch shapes (event batch, grid fill) on
+ * `fraction` of every scene's packets, tallying into mu_scratch (same shape as
+ * mu), and keeps the fastest for later launches. */
 int kp_batch_autotune( kp_batch_t * batch, const kp_transport_cfg_t * cfg, double fraction,
                        void * mu_scratch, void * stream, kp_tune_result_t * result );
 

@@ -43,7 +43,7 @@ struct kp_batch
     long long  * d_prefix_trial = nullptr;      // autotuner sample
     kp::scene_dev_t * d_scenes = nullptr;
     // launch shape (autotuned)
-    int threads = 128, lane_batch = 32, grid_pct = 100;
+    int lane_batch = 32, grid_pct = 100;
     // CUDA graph of the last launch configuration
     cudaGraphExec_t gexec = nullptr;
     kp::fwd_params_t gparams {  };
@@ -319,8 +319,7 @@ int kp_batch_autotune( kp_batch_t * b, const kp_transport_cfg_t * cfg, double fr
         cudaEvent_t e0, e1;
         KP_CUDA( cudaEventCreate( & e0 ) );
         KP_CUDA( cudaEventCreate( & e1 ) );
-        const int shapes[ ][ 3 ] = { { 128, 32, 100 }, { 128, 24, 100 }, { 128, 16, 100 },
-                                     { 128, 32, 80 }, { 128, 24, 80 } };
+        const int shapes[ ][ 2 ] = { { 32, 100 }, { 24, 100 }, { 16, 100 }, { 32, 80 }, { 24, 80 } };
         constexpr int n_shapes = ( int ) ( sizeof( shapes ) / sizeof( shapes[ 0 ] ) );
         float t_min[ n_shapes ];
         for( int i = 0; i < n_shapes; ++ i ) t_min[ i ] = 1e30f;
@@ -334,9 +333,8 @@ int kp_batch_autotune( kp_batch_t * b, const kp_transport_cfg_t * cfg, double fr
             for( int rep = 0; rep < 4; ++ rep )
                 for( int i = 0; i < n_shapes; ++ i )
                 {
-                    b->threads = shapes[ i ][ 0 ];
-                    b->lane_batch = shapes[ i ][ 1 ];
-                    b->grid_pct = shapes[ i ][ 2 ];
+                    b->lane_batch = shapes[ i ][ 0 ];
+                    b->grid_pct = shapes[ i ][ 1 ];
                     kp::fwd_params_t P;
                     make_batch_params( b, c, mu_scratch, nullptr, P, true );
                     KP_CUDA( cudaEventRecord( e0, s ) );
@@ -361,13 +359,12 @@ int kp_batch_autotune( kp_batch_t * b, const kp_transport_cfg_t * cfg, double fr
         for( int i = 1; i < n_shapes; ++ i )
             if( t_min[ i ] < t_min[ bi ] ) bi = i;
         const float best = t_min[ bi ];
-        b->threads = shapes[ bi ][ 0 ];
-        b->lane_batch = shapes[ bi ][ 1 ];
-        b->grid_pct = shapes[ bi ][ 2 ];
+        b->lane_batch = shapes[ bi ][ 0 ];
+        b->grid_pct = shapes[ bi ][ 1 ];
         if( b->gexec ) { cudaGraphExecDestroy( b->gexec ); b->gexec = nullptr; }
         if( res )
         {
-            res->threads = b->threads;
+            res->threads = kp::WALK_THREADS;
             res->lane_batch = b->lane_batch;
             res->grid_pct = b->grid_pct;
             res->sample_ms = best;

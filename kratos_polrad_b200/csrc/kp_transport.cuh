@@ -48,7 +48,8 @@ struct scene_dev_t
 #define KP_WALK_INNER_FLUX 2
 #endif
 
-// Packets of a warp's pool (kp_walk.cu).
+// k_walk's block, and the packets of a warp's pool (kp_walk.cu).
+constexpr int WALK_THREADS = 128;
 #ifndef KP_WALK_POOL
 #define KP_WALK_POOL 128
 #endif

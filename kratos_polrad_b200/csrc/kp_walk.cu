@@ -90,7 +90,7 @@ namespace
                                      // 9.06 against 8.39)
 #endif
 
-constexpr int WALK_THREADS = 128, WALK_WARPS = WALK_THREADS / 32;
+constexpr int WALK_WARPS = WALK_THREADS / 32;
 
 // How a flight ended; a list entry of an ended packet is its slot and this.
 enum end_kind { END_NONE = 0, END_ESCAPED = 1, END_LOST = 2, END_STEPS = 3, END_EVENT = 4 };
