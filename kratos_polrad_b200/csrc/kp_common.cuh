@@ -266,15 +266,15 @@ struct kp_mesh
     // Recomputes d_ext from d_sigma on stream s: every solve does this first,
     // since callers may write the coefficients through kp_mesh_sigma_ptr.
     void refresh_ext( cudaStream_t s );
-    // Gives back a buffer, or keeps it when a captured solve was given it; the
-    // other marks the buffers that a solve on s was given, if s is captured.
+    // Gives back a buffer, or keeps it when a captured solve was given it.
     void drop( void * p, bool & was_captured );
+    // Marks the buffers there are as given to a captured solve, if s is captured.
+    void note_capture( cudaStream_t s );
     // Memory that a solve cannot do without.  Where there is too little, the
     // mesh first gives back what is kept for speed alone: the packet pools, the
     // flux sums and an order that only the packet count asked for.  A solve
     // makes those last, as large as still fits.
     void need( void ** p, size_t bytes );
-    void note_capture( cudaStream_t s );
     void release_sort(  );
     void release(  );
 };

@@ -1412,10 +1412,14 @@ void ensure_peel_queue( kp_mesh_t * mesh, long long n_packets )
 // cell (kp_mesh_peel_order).  What the order saves is the march's L1 misses;
 // what it costs are four launches over the rays and the cells.  Solves as
 // queued and sorted: 9.3 MB of extinction (2-level clump) 66.1 and 68.9 ms per
-// 1e7 packets along x, 10.8 and 10.5 per 1e6 at inclination 60; 16 MB, a
-// gradient of 1e6 packets, 24.9 and 22.5; 20 MB 13.5 and 12.9; 32 MB 15.4 and
-// 14.6, and 1e5 packets 2.57 and 2.52, which the sort's buffers, about 1 ms on a
-// mesh's first such solve, outweigh; 51 MB 18.1 and 16.8; 74 MB 20.3 and 18.8.
+// 1e7 packets along x, 10.8 and 10.5 per 1e6 at inclination 60.  From 14 to
+// 31 MB (clumps and uniform meshes of 144 to 192 cells a side; 5e5, 1e6 and 4e6
+// packets) sorted is faster by 0 to 9% along x, 0 to 13% along z, 2 to 18% along
+// y, 1 to 6% at inclination 60 and between 1% slower and 3% faster obliquely; the
+// one exception is the 14 MB clump along x at 4e6 packets, 29.9 and 30.6 ms.  2e5
+// packets gain as much, 0.02 to 0.3 ms, but the sort's buffers take about 1 ms on
+// a mesh's first such solve: hence the packet count.  51 MB 18.1 and 16.8 ms; 74
+// MB 20.3 and 18.8.
 bool peel_sorted( const kp_mesh * mesh, long long n )
 {
     if( mesh->peel_order != KP_PEEL_ORDER_AUTO )

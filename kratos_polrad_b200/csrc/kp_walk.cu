@@ -4,7 +4,9 @@
 // (modules/particle/evolve/generate_par.h:51-62 -> ker_gen, then
 // evolve/integrator.h:47-63 -> ker_itg running photon::cart_t::proc) by one
 // persistent launch.  Each warp owns a pool of packets in global memory
-// (all pools together stay in L2) and works on it in three phases:
+// (48 MB at most together, of which the peel-off queue's stream evicts a part
+// from L2: 3.1 GB written and 1.4 GB read per 1e7 packets of the clump) and
+// works on it in three phases:
 //   walk    the lanes take ready packets and march each to the end of its
 //           flight: an interaction, the domain's boundary or a step limit;
 //   events  the interactions, 32 together: albedo, peel-off ray, roulette,
@@ -27,7 +29,7 @@
 // by selects, below, 5.6 ms).  Warp pools, fields in chunks of 32 and the
 // interaction's packet read again for its second half: 4.2 ms, against 6.0 ms
 // for the walk before.  With the extinction ahead (AHEAD, below), against the
-// walk before: the clump 5.96 -> 3.99 ms per 1e6 packets, 1.85 -> 1.44 ms per
+// walk before: the clump 5.96 -> 3.99 ms per 1e6 packets, 1.85 -> 1.36 ms per
 // 3e5, 0.56 -> 0.24 ms per 2000; the atmosphere 11.5 -> 8.5 ms per 1e6, 2.57 ->
 // 1.15 ms per 1117; the large scene 11.5 -> 8.0 ms per 2e6; the adjoint's replay
 // 4.49 -> 3.86 ms.
@@ -68,10 +70,12 @@ static_assert( sizeof( pool_chunk_t ) == 32 * 128, "pool chunk" );
 namespace
 {
 
-// Scheduling, times for 1e6 packets of the clump and of the atmosphere.
+// Scheduling, times for 1e6 packets of the clump and of the atmosphere (FETCH
+// and PARK: of the clump and of the large scene's 2e6).
 #ifndef KP_WALK_FETCH
-#define KP_WALK_FETCH 8              // idle lanes that wait for a fetch batch (4: 4.94
-                                     // against 4.95 ms, 9.62 against 9.63)
+#define KP_WALK_FETCH 8              // idle lanes that wait for a fetch batch (4 and 12:
+                                     // within 1%; 16: 4.00 against 3.97 ms, 8.40
+                                     // against 7.96)
 #endif
 #ifndef KP_WALK_HOP
 #define KP_WALK_HOP 6                // lanes that wait for a block hand-off (8: 4.20
@@ -82,7 +86,9 @@ namespace
                                      // 4.21 ms, 8.62 against 8.39)
 #endif
 #ifndef KP_WALK_PARK
-#define KP_WALK_PARK 20              // flights under way that may be put back
+#define KP_WALK_PARK 20              // flights under way that may be put back (8: 4.51
+                                     // against 3.97 ms, 8.55 against 7.96; 14: 4.08
+                                     // and 8.13; 26 and 32: within 1%)
 #endif
 #ifndef KP_WALK_MINB
 #define KP_WALK_MINB 5               // resident blocks the registers allow (96 registers;
