@@ -631,7 +631,7 @@ extern "C" int kp_transport_adjoint( kp_mesh_t * mesh, const kp_transport_cfg_t 
         // both marches read the queue in the forward solve's order
         int * perm = kp::march_order( mesh, P.n_packets, s );
         const kp::walk_pool_t pool( mesh->pool, std::min( chunk, P.n_packets ), s );
-        mesh->note_capture( s );
+        mesh->note_capture( s, true, true );
         static thread_local kp::fwd_params_t C;
         for( long long done = 0; done < P.n_packets; done += chunk )
         {
@@ -684,7 +684,7 @@ extern "C" int kp_transport_forward_tape( kp_mesh_t * mesh, const kp_transport_c
         auto s = ( cudaStream_t ) stream;
         const kp::walk_pool_t pool( mesh->pool, P.n_packets, s );
         kp::begin_flux( mesh, cfg->tally_mode, P, s );
-        mesh->note_capture( s );
+        mesh->note_capture( s, true, true );
         KP_CUDA( cudaMemsetAsync( P.work, 0, 4 * sizeof( unsigned long long ), s ) );
         KP_CUDA( cudaMemsetAsync( P.adj_head, 0xff, P.n_packets * sizeof( int ), s ) );
         KP_CUDA( cudaMemsetAsync( P.adj_flag, 0, P.n_packets * sizeof( int ), s ) );
@@ -723,7 +723,7 @@ extern "C" int kp_transport_adjoint_tape( kp_mesh_t * mesh, long long tape_id,
         P.pq_perm = mesh->tape_sorted ? mesh->d_sort_perm : nullptr;   // ... and order
         auto s = ( cudaStream_t ) stream;
         const kp::walk_pool_t pool( mesh->pool, mesh->tape_n, s );
-        mesh->note_capture( s );
+        mesh->note_capture( s, true, true );
         mesh->refresh_ext( s );
         const unsigned gs = 4 * 148;
         kp::k_adj_score<<< gs, 256, 0, s >>>( P );                        // G from the tape

@@ -268,8 +268,9 @@ struct kp_mesh
     void refresh_ext( cudaStream_t s );
     // Gives back a buffer, or keeps it when a captured solve was given it.
     void drop( void * p, bool & was_captured );
-    // Marks the buffers there are as given to a captured solve, if s is captured.
-    void note_capture( cudaStream_t s );
+    // Marks what a solve on s was given, if s is captured: the flux sums and the
+    // sort's buffers, the queue and its order (queue), the adjoint's (adj).
+    void note_capture( cudaStream_t s, bool queue, bool adj );
     // Memory that a solve cannot do without.  Where there is too little, the
     // mesh first gives back what is kept for speed alone: the packet pools, the
     // flux sums and an order that only the packet count asked for.  A solve

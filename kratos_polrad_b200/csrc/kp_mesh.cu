@@ -202,9 +202,12 @@ void kp_mesh::need( void ** p, size_t bytes )
     KP_CUDA( e );
 }
 
-void kp_mesh::note_capture( cudaStream_t s )
+void kp_mesh::note_capture( cudaStream_t s, bool queue, bool adj )
 {
-    if( kp::capturing( s ) ) pq_captured = perm_captured = adj_captured = sort_captured = true;
+    if( ! kp::capturing( s ) ) return;
+    sort_captured = true;
+    if( queue ) pq_captured = perm_captured = true;
+    if( adj )   adj_captured = true;
 }
 
 void kp_mesh::release_sort(  )

@@ -1569,7 +1569,7 @@ void launch_deferred( kp_mesh_t * mesh, fwd_params_t & P, cudaStream_t s )
     int * perm = march_order( mesh, P.n_packets, s );
     const walk_pool_t pool( mesh->pool, std::min( chunk, P.n_packets ), s );
     begin_flux( mesh, TALLY, P, s );
-    mesh->note_capture( s );
+    mesh->note_capture( s, true, false );
     static thread_local fwd_params_t C;
     for( long long done = 0; done < P.n_packets; done += chunk )
     {
@@ -1614,7 +1614,7 @@ extern "C" int kp_transport_forward( kp_mesh_t * mesh, const kp_transport_cfg_t 
             auto s = ( cudaStream_t ) stream;
             const kp::walk_pool_t pool( mesh->pool, P.n_packets, s );
             kp::begin_flux( mesh, cfg->tally_mode, P, s );
-            mesh->note_capture( s );
+            mesh->note_capture( s, false, false );
             KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
             kp::launch_walk( P, pool, cfg->tally_mode, kp::WALK_FORWARD, s );
             if( kp::split_event ) KP_CUDA( cudaEventRecord( kp::split_event, s ) );
@@ -1686,7 +1686,7 @@ void launch_resume_deferred( kp_mesh_t * mesh, fwd_params_t & P, cudaStream_t s 
     int * perm = march_order( mesh, items, s );
     const walk_pool_t pool( mesh->pool, std::min( chunk, items ), s );
     begin_flux( mesh, TALLY, P, s );
-    mesh->note_capture( s );
+    mesh->note_capture( s, true, false );
     static thread_local fwd_params_t C;
     for( long long lo = 0; lo < items; lo += chunk )
     {
@@ -1748,7 +1748,7 @@ extern "C" int kp_transport_forward_resume( kp_mesh_t * mesh, const kp_transport
             {
                 const kp::walk_pool_t pool( mesh->pool, P.n_packets + P.rs_n_in, s );
                 kp::begin_flux( mesh, cfg->tally_mode, P, s );
-                mesh->note_capture( s );
+                mesh->note_capture( s, false, false );
                 KP_CUDA( cudaMemsetAsync( P.work, 0, sizeof( unsigned long long ), s ) );
                 kp::launch_walk( P, pool, cfg->tally_mode, kp::WALK_FORWARD, s );
                 if( kp::split_event ) KP_CUDA( cudaEventRecord( kp::split_event, s ) );

@@ -267,6 +267,8 @@ void captured(  )
             solve_t s( n, kind != 3 );
             return kind == 2 ? s.adjoint( m, S ) : s.run( m, S );
         };
+        solve_t image( 20000, true );                // a queue and adjoint buffers beside it
+        expect( image.run( m, S ) == KP_OK && image.adjoint( m, S ) == KP_OK, "solve" );
         expect( solve( 20000 ) == KP_OK, "solve" );
         F.capturing = S;
         F.launches.clear(  );
@@ -280,6 +282,9 @@ void captured(  )
             if( k > 0 ) expect( F.live.size(  ) <= n_live, "outgrown buffers pile up" );
             n_live = F.live.size(  );
         }
+        solve_t larger( 500000, true );
+        expect( larger.adjoint( m, S ) == KP_OK, "larger solve" );
+        expect( m->kept.size(  ) == ( kind == 0 ? 1 : kind == 3 ? 0 : 2 ), "kept: what the capture was given, no more" );
         expect( kp_mesh_peel_queue_limit( m, 5000 ) == KP_OK && solve( 1000 ) == KP_OK, "lower limit" );
         for( uintptr_t a : held )
             expect( F.live.count( a ) != 0, "a captured solve's memory was freed" );
